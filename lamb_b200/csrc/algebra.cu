@@ -8,6 +8,7 @@
 #include <algorithm>
 
 #include "algebra.cuh"
+#include "panel.cuh"
 
 namespace lamb {
 
@@ -203,6 +204,7 @@ void move_matrix(Ctx* ctx, DevMatrix* dst, DevMatrix* src) {
   std::vector<float> pos = dst->h_pos;
   float box[3] = {dst->box[0], dst->box[1], dst->box[2]};
   std::vector<int32_t> ord = dst->h_order;
+  std::shared_ptr<GroupTab> rg = dst->rgrp, cg = dst->cgrp;
   free_matrix_buffers(ctx, dst);
   *dst = std::move(*src);
   *src = DevMatrix{};
@@ -211,7 +213,13 @@ void move_matrix(Ctx* ctx, DevMatrix* dst, DevMatrix* src) {
     dst->h_pos = pos;
     memcpy(dst->box, box, sizeof(box));
   }
-  if (dst->h_order.empty() && (int)ord.size() == dst->n_rows) dst->h_order = ord;
+  if (dst->h_order.empty() && (int)ord.size() == dst->n_rows) {
+    dst->h_order = ord;
+    if (!dst->rgrp && !dst->cgrp && rg && cg && rg->n_atoms == dst->n_rows && cg->n_atoms == dst->n_cols) {
+      dst->rgrp = rg;
+      dst->cgrp = cg;
+    }
+  }
 }
 
 int32_t axpby_impl(Ctx* ctx, double alpha, DevMatrix* X, double beta, DevMatrix* Y) {
@@ -251,6 +259,8 @@ int32_t copy_impl(Ctx* ctx, const DevMatrix* X, DevMatrix* Y) {
   tmp.h_pos = X->h_pos;
   memcpy(tmp.box, X->box, sizeof(tmp.box));
   tmp.h_order = X->h_order;
+  tmp.rgrp = X->rgrp;
+  tmp.cgrp = X->cgrp;
   LAMB_TRY(upload_block_sizes(ctx, &tmp));
   LAMB_TRY(dalloc(ctx, &tmp.row_p, tmp.n_rows + 1));
   LAMB_TRY(dalloc(ctx, &tmp.col, std::max<int64_t>(tmp.nnz, 1)));

@@ -19,6 +19,8 @@ namespace lamb {
 // ---- status codes (level/type pairs of src/lamb_error.F90:120-159) -------
 inline int32_t make_status(int level, int type) { return level * 100000 + (type + 50000); }
 
+struct GroupTab;
+
 // ---- device matrix ------------------------------------------------------------
 // Every device matrix is one block-CSR over "sector order": the atoms of
 // subset 1 first (in local order), then subset 2, ... along rows and columns.
@@ -42,7 +44,7 @@ struct DevMatrix {
   int64_t* off = nullptr;      // [nnz], 0-based data offset of each block
   double* data = nullptr;      // [data_len]
   int64_t data_cap = 0;        // elements of data a later multiply into this matrix may reuse (0: none)
-  double* norms = nullptr;     // [nnz] Frobenius norms, valid when norms_valid
+  double* norms = nullptr;     // [nnz] Frobenius norms, then their range (NormRange), valid when norms_valid
   bool norms_valid = false;
   // Locality: optional row-atom coordinates (sector order) and the processing
   // order of rows derived from them (Morton) or from the pattern (Cuthill-McKee).
@@ -50,6 +52,8 @@ struct DevMatrix {
   float box[3] = {0, 0, 0};
   std::vector<int32_t> h_order;  // row processing order, empty until computed
   int32_t* order = nullptr;      // device copy of h_order
+  // Groups of row and column atoms for the panel products (panel.cuh), empty until needed.
+  std::shared_ptr<GroupTab> rgrp, cgrp;
   // Result of a multiply computed in row chunks: the data of chunk p in
   // sector s is [chunk_rng[2*(p*S_all+s)], chunk_rng[2*(p*S_all+s)+1]) relative
   // to the sector's base; chunk p is complete when the context's chunk_ev[p]
@@ -76,6 +80,7 @@ enum ScratchSlot : int { kScrEnt = 0, kScrWork, kScrWorkC, kScrPlaneA, kScrPlane
 
 struct Ctx {
   int device = 0;
+  size_t total_mem = 0;  // of the device
   cudaStream_t stream = nullptr;
   std::string last_error;
   std::map<int64_t, std::unique_ptr<DevMatrix>> mats;
@@ -104,7 +109,23 @@ struct Ctx {
   cudaEvent_t kern_ev[2][kMaxChunks] = {};
   int kern_chunks = 0;
   cudaStream_t copy_stream = nullptr;
+  // Pinned host memory for the small results a call waits for (norm ranges,
+  // panel totals); every user waits for the stream before it reads.
+  int64_t* pin = nullptr;
+  int* tile_err = nullptr;  // device: set by the panel kernel when one of its bounded waits ran out
 };
+// Words of the pinned buffer.
+constexpr int kPinCount = 0;    // what the symbolic count leaves (CountStat, 5 words)
+constexpr int kPinPanel = 5;    // panel totals
+constexpr int kPinTileErr = 8;  // tile_err after the last panel product
+constexpr int kPinWords = 64;
+// The smallest and the largest of a matrix's block norms, as bit patterns that
+// an atomic maximum can collect (norms are >= 0 or NaN; a NaN is the largest).
+struct NormRange {
+  unsigned long long not_min, max;
+};
+// Reports (once) that a panel product stopped; the stream has been waited for.
+int32_t check_tiles(Ctx* ctx);
 
 // Completes a pending result filter (waits for its counts and updates the
 // matrix's host metadata).  Every entry point reaches it through get_matrix.
@@ -196,8 +217,6 @@ int32_t inclusive_scan_i64(Ctx* ctx, const int64_t* in, int64_t* out, int64_t n)
 int32_t sum_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out);
 // Largest of n int64 (waits for the stream); 0 when n == 0.
 int32_t max_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out);
-// Smallest of n doubles (waits for the stream); 0 when n == 0.
-int32_t min_f64(Ctx* ctx, const double* in, int64_t n, double* host_out);
 
 // ---- device helpers -------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v) {

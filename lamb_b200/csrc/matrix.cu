@@ -15,6 +15,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "panel.cuh"
 
 namespace lamb {
 
@@ -76,6 +77,15 @@ void trace_mark(Ctx* ctx, const char* what) {
   ctx->trace_t = now;
 }
 
+int32_t check_tiles(Ctx* ctx) {
+  const int code = (int)*(volatile int*)&ctx->pin[kPinTileErr];
+  if (!code) return LAMB_GPU_OK;
+  ctx->pin[kPinTileErr] = 0;
+  LAMB_CUDA(ctx, cudaMemsetAsync(ctx->tile_err, 0, sizeof(int), ctx->stream));
+  return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_INTERNAL_ERROR,
+              "panel product stopped: a wait ran out (code " + std::to_string(code) + ")");
+}
+
 int32_t settle(Ctx* ctx) {
   DevMatrix* m = ctx->pend_m;
   if (!m) return LAMB_GPU_OK;
@@ -86,7 +96,7 @@ int32_t settle(Ctx* ctx) {
   int64_t tot = 0;
   for (int64_t x : m->sec_nblk) tot += x;
   m->nnz = tot;
-  return LAMB_GPU_OK;
+  return check_tiles(ctx);
 }
 
 DevMatrix* find_matrix(Ctx* ctx, lamb_gpu_matrix h) {
@@ -116,6 +126,8 @@ void free_matrix_buffers(Ctx* ctx, DevMatrix* m) {
   dfree(ctx, m->norms);
   dfree(ctx, m->order);
   m->h_order.clear();
+  m->rgrp.reset();
+  m->cgrp.reset();
   m->norms_valid = false;
   m->n_chunks = 0;
   m->chunk_rng.clear();
@@ -217,48 +229,47 @@ int32_t max_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out) {
   return LAMB_GPU_OK;
 }
 
-int32_t min_f64(Ctx* ctx, const double* in, int64_t n, double* host_out) {
-  *host_out = 0.0;
-  if (n <= 0) return LAMB_GPU_OK;
-  double* d_out = nullptr;
-  LAMB_TRY(dalloc(ctx, &d_out, 1));
-  size_t bytes = 0;
-  LAMB_CUDA(ctx, cub::DeviceReduce::Min(nullptr, bytes, in, d_out, n, ctx->stream));
-  void* tmp = nullptr;
-  LAMB_TRY(dalloc(ctx, (char**)&tmp, (int64_t)bytes + 16));
-  cudaError_t e = cub::DeviceReduce::Min(tmp, bytes, in, d_out, n, ctx->stream);
-  cudaFreeAsync(tmp, ctx->stream);
-  LAMB_CUDA(ctx, e);
-  LAMB_CUDA(ctx, cudaMemcpyAsync(host_out, d_out, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  dfree(ctx, d_out);
-  return LAMB_GPU_OK;
-}
-
 // ---- block norms -----------------------------------------------------------------------
 // One warp per block row; each lane sums whole blocks sequentially (fixed order).
 __global__ void k_block_norms(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
                               const int64_t* __restrict__ off, const int8_t* __restrict__ row_bs,
                               const int8_t* __restrict__ col_bs, const double* __restrict__ data,
-                              double* __restrict__ norms) {
+                              double* __restrict__ norms, unsigned long long* __restrict__ range) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  // norms are >= 0 or NaN: their bit patterns order like the values, any NaN above infinity
+  unsigned long long lo = 0ull, hi = 0ull;  // largest complement of a pattern, largest pattern
   for (int64_t r = warp; r < n_rows; r += nwarps) {
     const int bi = row_bs[r];
     for (int64_t b = row_p[r] + lane; b < row_p[r + 1]; b += 32) {
       const int64_t n = (int64_t)bi * col_bs[col[b]];
-      norms[b] = block_norm_seq(data + off[b], n);
+      const double v = block_norm_seq(data + off[b], n);
+      norms[b] = v;
+      const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+      lo = max(lo, ~u);
+      hi = max(hi, u);
     }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0 && lo) {
+    atomicMax(&range[0], lo);
+    atomicMax(&range[1], hi);
   }
 }
 
 int32_t ensure_norms(Ctx* ctx, DevMatrix* m) {
   if (m->norms_valid) return LAMB_GPU_OK;
-  if (!m->norms) LAMB_TRY(dalloc(ctx, &m->norms, std::max<int64_t>(m->nnz, 1)));
+  if (!m->norms) LAMB_TRY(dalloc(ctx, &m->norms, m->nnz + 2));
+  unsigned long long* range = reinterpret_cast<unsigned long long*>(m->norms + m->nnz);
+  LAMB_CUDA(ctx, cudaMemsetAsync(range, 0, 2 * sizeof(*range), ctx->stream));
   if (m->nnz > 0) {
     k_block_norms<<<grid_for((int64_t)m->n_rows * 32), kThreads, 0, ctx->stream>>>(
-        m->n_rows, m->row_p, m->col, m->off, m->row_bs, m->col_bs, m->data, m->norms);
+        m->n_rows, m->row_p, m->col, m->off, m->row_bs, m->col_bs, m->data, m->norms, range);
     LAMB_LAUNCHED(ctx);
   }
   m->norms_valid = true;
@@ -622,6 +633,7 @@ int32_t lamb_gpu_ctx_create(int32_t device, lamb_gpu_ctx** out) {
   if (cudaSetDevice(device) != cudaSuccess) return make_status(LAMB_LEVEL_FAILURE, LAMB_TYPE_EXTERNAL_ERROR);
   auto* ctx = new Ctx;
   ctx->device = device;
+  ctx->total_mem = p.totalGlobalMem;
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete ctx;
     return make_status(LAMB_LEVEL_FAILURE, LAMB_TYPE_EXTERNAL_ERROR);
@@ -631,6 +643,17 @@ int32_t lamb_gpu_ctx_create(int32_t device, lamb_gpu_ctx** out) {
   for (auto& row : ctx->kern_ev)
     for (auto& ev : row) cudaEventCreate(&ev);
   cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
+  if (cudaMallocHost(&ctx->pin, sizeof(int64_t) * kPinWords) != cudaSuccess ||
+      cudaMalloc(&ctx->tile_err, sizeof(int)) != cudaSuccess ||
+      cudaMemset(ctx->tile_err, 0, sizeof(int)) != cudaSuccess) {
+    cudaFreeHost(ctx->pin);
+    cudaFree(ctx->tile_err);
+    cudaStreamDestroy(ctx->copy_stream);
+    cudaStreamDestroy(ctx->stream);
+    delete ctx;
+    return make_status(LAMB_LEVEL_MEMORY, LAMB_TYPE_EXTERNAL_ERROR);
+  }
+  ctx->pin[kPinTileErr] = 0;
   if (const char* t = std::getenv("LAMB_GPU_TRACE")) {
     ctx->trace = t[0] == '1' || t[0] == '2';
     ctx->trace_host = t[0] == '2';
@@ -661,6 +684,8 @@ int32_t lamb_gpu_ctx_destroy(lamb_gpu_ctx* c) {
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   if (ctx->pend_ev) cudaEventDestroy(ctx->pend_ev);
   if (ctx->pend_h) cudaFreeHost(ctx->pend_h);
+  cudaFreeHost(ctx->pin);
+  cudaFree(ctx->tile_err);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return LAMB_GPU_OK;
@@ -687,7 +712,7 @@ int32_t lamb_gpu_ctx_synchronize(lamb_gpu_ctx* c) {
   auto* ctx = reinterpret_cast<Ctx*>(c);
   if (!ctx) return make_status(LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS);
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return LAMB_GPU_OK;
+  return check_tiles(ctx);
 }
 
 int32_t lamb_gpu_matrix_upload(lamb_gpu_ctx* c, const lamb_c_sector* sec, int32_t n_sec, lamb_gpu_matrix* handle) {
@@ -833,6 +858,8 @@ int32_t lamb_gpu_matrix_set_positions(lamb_gpu_ctx* c, lamb_gpu_matrix h, const 
   memcpy(m->box, box, sizeof(m->box));
   m->h_order.clear();
   dfree(ctx, m->order);
+  m->rgrp.reset();  // the groups' ranks follow the order
+  m->cgrp.reset();
   return LAMB_GPU_OK;
 }
 
@@ -941,6 +968,7 @@ int32_t lamb_gpu_matrix_download(lamb_gpu_ctx* c, lamb_gpu_matrix h, lamb_c_sect
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->copy_stream));
   free_sector_index(ctx, &si);
+  LAMB_TRY(check_tiles(ctx));
   for (int a = 0; a < m->n_rsub; ++a)
     for (int b = 0; b < S; ++b) {
       auto& o = out[a * S + b];

@@ -59,6 +59,7 @@
 
 #include "lamb_probe.h"
 #include "multiply.cuh"
+#include "ptx.cuh"
 
 namespace lamb {
 namespace tc {
@@ -173,45 +174,11 @@ struct TcArgs {
 };
 
 // ---- PTX helpers -----------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
 // x * 2^e for any e, out of line: the scatter loop is unrolled 64 times and
 // only exponents beyond kExactExp (not met in practice) take this path.
 __device__ __noinline__ double scale_wide(double x, int e) { return ldexp(x, e); }
 // 2^e for -1022 <= e <= 1023, exactly.
 __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
-__device__ __forceinline__ uint64_t now_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void bar_init(unsigned long long* b, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(unsigned long long* b) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(b)) : "memory");
-}
-__device__ __forceinline__ bool bar_try(unsigned long long* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// try_wait with a suspend-time hint: a waiting thread sleeps in hardware
-// (issuing nothing) until the phase completes or about `ns` nanoseconds pass.
-__device__ __forceinline__ bool bar_try_sleep(unsigned long long* b, uint32_t parity, uint32_t ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity), "r"(ns)
-      : "memory");
-  return ok != 0;
-}
 // Waits until the phase with the given parity has completed; gives up after
 // 2 s (or when another role aborted), recording `code`.  The waiting thread
 // sleeps between checks, leaving the issue slots to the other warps of its

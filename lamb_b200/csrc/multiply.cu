@@ -15,6 +15,7 @@
 #include <numeric>
 
 #include "multiply.cuh"
+#include "panel.cuh"
 
 namespace lamb {
 
@@ -26,6 +27,8 @@ void free_symbolic(Ctx* ctx, Symbolic& s) {
     dfree(ctx, s.ent);
   dfree(ctx, s.ids);
   dfree(ctx, s.c_row);
+  dfree(ctx, s.c_bm);
+  dfree(ctx, s.c_pre);
 }
 
 int32_t check_compatible(Ctx* ctx, const DevMatrix* A, const DevMatrix* B) {
@@ -40,30 +43,46 @@ int32_t check_compatible(Ctx* ctx, const DevMatrix* A, const DevMatrix* B) {
 // reached by surviving products A_ik.B_kj (|A_ik|*|B_kj| >= eps).
 constexpr int kSymThreads = 256;
 
-// FILT = false when no product can fall below eps: the norms are then not read.
-template <bool FILT>
-__device__ __forceinline__ bool keep_pair(double na, const double* __restrict__ b_nrm, int64_t bb, double eps) {
-  return !FILT || !(na * b_nrm[bb] < eps);
+// No product falls below eps when the smallest norms of A and B multiply to
+// at least eps (fl(x*y) is monotone in x and y); any NaN norm keeps the test.
+__host__ __device__ inline double bits_to_double(unsigned long long u) {
+  double d;
+  memcpy(&d, &u, sizeof(d));
+  return d;
 }
-// The fill always reads the norms (with eps = 0 when nothing is filtered:
+__host__ __device__ inline bool finite_norms(const NormRange& r) { return r.max < 0x7ff0000000000000ull; }
+__host__ __device__ inline bool filter_acts(const NormRange& a, const NormRange& b, double eps) {
+  return !finite_norms(a) || !finite_norms(b) || !(bits_to_double(~a.not_min) * bits_to_double(~b.not_min) >= eps);
+}
+// What the host needs of the count kernel beside the rows' counts.
+struct CountStat {
+  NormRange a, b;
+  unsigned long long max_a_len;
+};
+// The count kernel does not read the norms when no product can fall below
+// eps.  The fill always reads the norms (with eps = 0 when nothing is filtered:
 // norms are >= 0 or NaN, so every pair stays); its norm-free variant measured
 // 1.4 ms slower at 6,144 waters while the count kernel gains 0.8 ms.
 __device__ __forceinline__ bool keep_norms(double na, double nb, double eps) { return !(na * nb < eps); }
 
-template <bool FILT>
 __global__ void __launch_bounds__(kSymThreads) k_sym_count(
     int32_t n_rows, const int64_t* __restrict__ a_row_p, const int32_t* __restrict__ a_col,
     const double* __restrict__ a_nrm, const int64_t* __restrict__ b_row_p, const int32_t* __restrict__ b_col,
     const double* __restrict__ b_nrm, const int8_t* __restrict__ row_bs, const int8_t* __restrict__ k_bs,
-    const int8_t* __restrict__ col_bs, double eps, int32_t n_words, int64_t* __restrict__ c_cnt,
-    int64_t* __restrict__ s_cnt, int64_t* __restrict__ p_cnt, double* __restrict__ row_flops,
-    unsigned* __restrict__ max_a_len) {
+    const int8_t* __restrict__ col_bs, double eps, int want_filt, const NormRange* __restrict__ range_a,
+    const NormRange* __restrict__ range_b, int32_t n_words, int64_t* __restrict__ c_cnt, int64_t* __restrict__ s_cnt, int64_t* __restrict__ p_cnt, double* __restrict__ row_flops,
+    CountStat* __restrict__ stat) {
   extern __shared__ uint32_t bm[];
   typedef cub::BlockReduce<int64_t, kSymThreads> RI;
   typedef cub::BlockReduce<double, kSymThreads> RD;
   __shared__ typename RI::TempStorage ti;
   __shared__ typename RD::TempStorage td;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kSymThreads / 32;
+  const bool filt = want_filt && filter_acts(*range_a, *range_b, eps);
+  if (blockIdx.x == 0 && tid == 0) {
+    stat->a = *range_a;
+    stat->b = *range_b;
+  }
   for (int64_t i = blockIdx.x; i < n_rows; i += gridDim.x) {
     for (int w = tid; w < n_words; w += kSymThreads) bm[w] = 0u;
     __syncthreads();
@@ -72,12 +91,12 @@ __global__ void __launch_bounds__(kSymThreads) k_sym_count(
     const int bi = row_bs[i];
     for (int64_t ab = a_row_p[i] + warp; ab < a_row_p[i + 1]; ab += nw) {
       const int k = a_col[ab];
-      const double na = FILT ? a_nrm[ab] : 0.0;
+      const double na = filt ? a_nrm[ab] : 0.0;
       const int bk = k_bs[k];
       const int64_t b1 = b_row_p[k + 1];
       for (int64_t bb = b_row_p[k] + lane; bb < b1; bb += 32) {
         ++pairs;
-        if (!keep_pair<FILT>(na, b_nrm, bb, eps)) continue;
+        if (filt && !keep_norms(na, b_nrm[bb], eps)) continue;
         const int j = b_col[bb];
         atomicOr(&bm[j >> 5], 1u << (j & 31));
         ++kept;
@@ -99,7 +118,7 @@ __global__ void __launch_bounds__(kSymThreads) k_sym_count(
       s_cnt[i] = tot_kept;
       p_cnt[i] = tot_pairs;
       row_flops[i] = tot_fl;
-      atomicMax(max_a_len, (unsigned)(a_row_p[i + 1] - a_row_p[i]));
+      atomicMax(&stat->max_a_len, (unsigned long long)(a_row_p[i + 1] - a_row_p[i]));
     }
     __syncthreads();
   }
@@ -139,7 +158,7 @@ __global__ void __launch_bounds__(kSymThreads) k_sym_pattern(
     int32_t n_rows, const int64_t* __restrict__ a_row_p, const int32_t* __restrict__ a_col,
     const double* __restrict__ a_nrm, const int64_t* __restrict__ b_row_p, const int32_t* __restrict__ b_col,
     const double* __restrict__ b_nrm, double eps, int32_t n_words, const int64_t* __restrict__ c_row_p,
-    int32_t* __restrict__ c_col) {
+    int32_t* __restrict__ c_col, uint32_t* __restrict__ g_bm, int32_t* __restrict__ g_pre) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t* bm = reinterpret_cast<uint32_t*>(smem_raw);
   int* wpre = reinterpret_cast<int*>(bm + n_words);
@@ -164,6 +183,10 @@ __global__ void __launch_bounds__(kSymThreads) k_sym_pattern(
     for (int w = tid; w < n_words; w += kSymThreads) {
       uint32_t bits = bm[w];
       int p = wpre[w];
+      if (g_bm) {
+        g_bm[i * n_words + w] = bits;
+        g_pre[i * n_words + w] = p;
+      }
       while (bits) {
         const int b = __ffs(bits) - 1;
         bits &= bits - 1u;
@@ -344,32 +367,24 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
   LAMB_TRY(dalloc(ctx, &s_cnt, std::max(n_rows, 1)));
   LAMB_TRY(dalloc(ctx, &p_cnt, std::max(n_rows, 1)));
   LAMB_TRY(dalloc(ctx, &rfl, std::max(n_rows, 1)));
-  unsigned* d_max_na = nullptr;
-  LAMB_TRY(dalloc(ctx, &d_max_na, 1));
-  LAMB_CUDA(ctx, cudaMemsetAsync(d_max_na, 0, sizeof(unsigned), ctx->stream));
-  // No product falls below eps when the smallest norms of A and B multiply to
-  // at least eps (fl(x*y) is monotone in x and y): the count kernel then
-  // skips the norm loads.  Any NaN norm keeps the test.
-  bool count_filt = filt;
-  if (filt && A->nnz && B->nnz) {
-    double min_a = 0.0, min_b = 0.0;
-    LAMB_TRY(min_f64(ctx, A->norms, A->nnz, &min_a));
-    LAMB_TRY(min_f64(ctx, B->norms, B->nnz, &min_b));
-    if (min_a * min_b >= eps) count_filt = false;
-  }
+  CountStat* d_stat = nullptr;
+  LAMB_TRY(dalloc(ctx, &d_stat, 1));
+  LAMB_CUDA(ctx, cudaMemsetAsync(d_stat, 0, sizeof(CountStat), ctx->stream));
+  auto range = [](const DevMatrix* m) { return reinterpret_cast<const NormRange*>(m->norms + m->nnz); };
+  static_assert(sizeof(CountStat) <= 8 * (kPinPanel - kPinCount), "pinned words of the count");
   const double fill_eps = filt ? eps : 0.0;
   const size_t smem_count = sizeof(uint32_t) * (size_t)std::max(n_words, 1);
   if (smem_count > 200 * 1024)
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "too many block columns for the symbolic bitmap");
   if (n_rows > 0) {
-    auto count_kern = count_filt ? k_sym_count<true> : k_sym_count<false>;
+    auto count_kern = k_sym_count;
     if (smem_count > 48 * 1024)
       LAMB_CUDA(ctx, cudaFuncSetAttribute(count_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
     int grid = 1;
     LAMB_TRY(resident_grid(ctx, count_kern, smem_count, n_rows, &grid));
     count_kern<<<grid, kSymThreads, smem_count, ctx->stream>>>(
-        n_rows, A->row_p, A->col, A->norms, B->row_p, B->col, B->norms, C->row_bs, B->row_bs, C->col_bs, eps,
-        n_words, c_cnt, s_cnt, p_cnt, rfl, d_max_na);
+        n_rows, A->row_p, A->col, A->norms, B->row_p, B->col, B->norms, C->row_bs, B->row_bs, C->col_bs, eps, filt,
+        range(A), range(B), n_words, c_cnt, s_cnt, p_cnt, rfl, d_stat);
     LAMB_LAUNCHED(ctx);
   }
   unsigned max_na = 0;
@@ -381,8 +396,14 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     LAMB_CUDA(ctx, cudaMemcpyAsync(h_s.data(), s_cnt, sizeof(int64_t) * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
     LAMB_CUDA(ctx, cudaMemcpyAsync(h_p.data(), p_cnt, sizeof(int64_t) * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
     LAMB_CUDA(ctx, cudaMemcpyAsync(h_f.data(), rfl, sizeof(double) * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
-    LAMB_CUDA(ctx, cudaMemcpyAsync(&max_na, d_max_na, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    LAMB_CUDA(ctx, cudaMemcpyAsync(ctx->pin + kPinCount, d_stat, sizeof(CountStat), cudaMemcpyDeviceToHost, ctx->stream));
     LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  }
+  if (n_rows) {
+    const CountStat& h = *reinterpret_cast<const CountStat*>(ctx->pin + kPinCount);
+    max_na = (unsigned)h.max_a_len;
+    out->filter_acts = filt && filter_acts(h.a, h.b, eps);
+    out->finite = finite_norms(h.a) && finite_norms(h.b);
   }
   trace_mark(ctx, "symbolic count");
   std::vector<int64_t> h_crp(n_rows + 1, 0), h_srb(n_rows + 1, 0);
@@ -431,10 +452,15 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     const size_t smem_pat = sizeof(uint32_t) * 2 * (size_t)std::max(n_words, 1);
     if (smem_pat > 48 * 1024)
       LAMB_CUDA(ctx, cudaFuncSetAttribute(k_sym_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_pat));
+    if (out->want_bits) {
+      LAMB_TRY(dalloc(ctx, &out->c_bm, (int64_t)n_rows * n_words));
+      LAMB_TRY(dalloc(ctx, &out->c_pre, (int64_t)n_rows * n_words));
+    }
     int pgrid = 1;
     LAMB_TRY(resident_grid(ctx, k_sym_pattern, smem_pat, n_rows, &pgrid));
     k_sym_pattern<<<pgrid, kSymThreads, smem_pat, ctx->stream>>>(n_rows, A->row_p, A->col, A->norms, B->row_p, B->col,
-                                                                B->norms, fill_eps, n_words, C->row_p, C->col);
+                                                                B->norms, fill_eps, n_words, C->row_p, C->col,
+                                                                out->c_bm, out->c_pre);
     LAMB_LAUNCHED(ctx);
   } else if (smem_fill > 220 * 1024) {
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "C block row too long for the symbolic fill");
@@ -470,7 +496,7 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     C->data_cap = need;
   }
   dfree(ctx, c_cnt); dfree(ctx, s_cnt); dfree(ctx, p_cnt); dfree(ctx, rfl); dfree(ctx, s_row_base);
-  dfree(ctx, d_max_na);
+  dfree(ctx, d_stat);
   trace_mark(ctx, "C data allocation");
   return LAMB_GPU_OK;
 }
@@ -661,6 +687,41 @@ int32_t result_filter(Ctx* ctx, DevMatrix* C, const double* c_nrm, double eps) {
 // the largest single C row's entries when that is more (a row is not split).
 constexpr int64_t kStackCapEntries = 1ll << 27;
 
+// Download ranges of C's row chunks: chunk p holds the rows at processing
+// positions q[p] .. q[p + 1] - 1 (order `ord`), inside every sector one range.
+static void chunk_ranges(DevMatrix* C, const Symbolic& sym, const std::vector<int32_t>& ord, const std::vector<int>& q) {
+  const int n = C->n_rows, S = C->n_csub, R = C->n_rsub, P = (int)q.size() - 1;
+  const size_t n_sec = (size_t)R * S;
+  std::vector<int32_t> sub_of(n);
+  for (int a = 0; a < R; ++a)
+    for (int r = C->rsub_base[a]; r < C->rsub_base[a + 1]; ++r) sub_of[r] = a;
+  std::vector<int64_t> before((size_t)(P + 1) * R, 0);  // rows of subset a at positions < q[p]
+  {
+    std::vector<int64_t> cnt(R, 0);
+    int p = 0;
+    for (int w = 0; w <= n; ++w) {
+      while (p <= P && q[p] == w) {
+        for (int a = 0; a < R; ++a) before[(size_t)p * R + a] = cnt[a];
+        ++p;
+      }
+      if (w < n) ++cnt[sub_of[ord[w]]];
+    }
+  }
+  C->chunk_rng.assign(2 * (size_t)P * n_sec, 0);
+  for (int p = 0; p < P; ++p)
+    for (int a = 0; a < R; ++a)
+      for (int b = 0; b < S; ++b) {
+        const size_t s2 = (size_t)a * S + b;
+        const int64_t cnt_a = C->rsub_cnt[a];
+        auto at = [&](int64_t rank) -> int64_t {  // data offset in the sector before local rank `rank`
+          if (rank >= cnt_a) return C->sec_dlen[s2];
+          return sym.h_base[(size_t)C->rsub_base[a] * S + (size_t)b * cnt_a + rank] - C->sec_base[s2];
+        };
+        C->chunk_rng[2 * ((size_t)p * n_sec + s2)] = at(before[(size_t)p * R + a]);
+        C->chunk_rng[2 * ((size_t)p * n_sec + s2) + 1] = at(before[(size_t)(p + 1) * R + a]);
+      }
+}
+
 // The rows, in processing order, are cut into chunks: first into kMinChunks
 // of about equal C-block count (downloads copy a chunk as soon as it is
 // done), then wherever a chunk would hold more than the stack cap.  Per chunk
@@ -742,37 +803,7 @@ static int32_t numeric_chunks(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C
     for (int w = q[p]; w < q[p + 1]; ++w) acc += sym.h_row_len[ord[w]];
     item[p + 1] = item[p] + acc;
   }
-  // ---- download ranges of every chunk in every sector ----
-  if (layout_ok) {
-    std::vector<int32_t> sub_of(n);
-    for (int a = 0; a < R; ++a)
-      for (int r = C->rsub_base[a]; r < C->rsub_base[a + 1]; ++r) sub_of[r] = a;
-    std::vector<int64_t> before((size_t)(P + 1) * R, 0);  // rows of subset a at positions < q[p]
-    {
-      std::vector<int64_t> cnt(R, 0);
-      int p = 0;
-      for (int w = 0; w <= n; ++w) {
-        while (p <= P && q[p] == w) {
-          for (int a = 0; a < R; ++a) before[(size_t)p * R + a] = cnt[a];
-          ++p;
-        }
-        if (w < n) ++cnt[sub_of[ord[w]]];
-      }
-    }
-    C->chunk_rng.assign(2 * (size_t)P * n_sec, 0);
-    for (int p = 0; p < P; ++p)
-      for (int a = 0; a < R; ++a)
-        for (int b = 0; b < S; ++b) {
-          const size_t s2 = (size_t)a * S + b;
-          const int64_t cnt_a = C->rsub_cnt[a];
-          auto at = [&](int64_t rank) -> int64_t {  // data offset in the sector before local rank `rank`
-            if (rank >= cnt_a) return C->sec_dlen[s2];
-            return sym.h_base[(size_t)C->rsub_base[a] * S + (size_t)b * cnt_a + rank] - C->sec_base[s2];
-          };
-          C->chunk_rng[2 * ((size_t)p * n_sec + s2)] = at(before[(size_t)p * R + a]);
-          C->chunk_rng[2 * ((size_t)p * n_sec + s2) + 1] = at(before[(size_t)(p + 1) * R + a]);
-        }
-  }
+  if (layout_ok) chunk_ranges(C, sym, ord, q);
   // ---- buffers ----
   Ent* ent = nullptr;
   Work* work = nullptr;
@@ -827,6 +858,55 @@ static int32_t numeric_chunks(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C
   return LAMB_GPU_OK;
 }
 
+// ---- FP64 numeric phase on group tiles -------------------------------------------------
+// Whether the panel kernel may be considered: its block sizes, and about half a
+// million block products (below that the launches that prepare the panels, some
+// 60 us, cost more than the stacks: 48 atoms of 0 to 3 rows, 53,000 products,
+// 625 us a call with stacks, 690 us with panels; 64 waters, 1.6 million, even).
+static bool panel_ok(const DevMatrix* A, const DevMatrix* B) {
+  return A->n_cols > 0 && (double)A->nnz * B->nnz >= (double)(1 << 19) * A->n_cols &&
+         panel_shapes_ok(A->h_row_bs, A->h_col_bs, B->h_col_bs);
+}
+
+// Groups of C's columns: A's when B lives on the same atoms (both then describe
+// the same runs), B's own otherwise.
+static int32_t product_groups(Ctx* ctx, DevMatrix* A, DevMatrix* B, std::shared_ptr<GroupTab>* cols) {
+  LAMB_TRY(ensure_groups(ctx, A));
+  if (A->h_row_bs == A->h_col_bs && B->h_row_bs == A->h_row_bs && B->h_col_bs == A->h_row_bs) {
+    *cols = A->rgrp;
+    return LAMB_GPU_OK;
+  }
+  LAMB_TRY(ensure_groups(ctx, B));
+  *cols = B->cgrp;
+  return LAMB_GPU_OK;
+}
+
+// The tile kernel, in kMinChunks launches when a download may overlap them.
+// *ran = false (nothing done) when the panels do not fit.
+static int32_t numeric_panel(Ctx* ctx, DevMatrix* A, DevMatrix* C, const Symbolic& sym, PanelPair* pair, double eps,
+                             double* c_nrm, bool overlap, bool* ran) {
+  C->n_chunks = 0;
+  C->chunk_rng.clear();
+  LAMB_TRY(panel_pack(ctx, pair, ctx->pin + kPinPanel, sym.filter_acts, ran));
+  if (!*ran) return LAMB_GPU_OK;
+  const int n = C->n_rows;
+  const bool layout_ok = (int)A->h_order.size() == n && (int64_t)C->h_order.size() == n &&
+                         (int64_t)sym.h_base.size() == (int64_t)n * C->n_csub;
+  std::vector<int32_t> done;
+  // the tile kernel skips blocks without elements
+  if (c_nrm) LAMB_CUDA(ctx, cudaMemsetAsync(c_nrm, 0, sizeof(double) * sym.c_nnz, ctx->stream));
+  LAMB_TRY(panel_tiles(ctx, *pair, C, sym.c_bm, sym.c_pre, c_nrm, sym.filter_acts, eps, overlap && layout_ok ? kMinChunks : 1, &done));
+  if (layout_ok) {
+    std::vector<int> q(1, 0);
+    q.insert(q.end(), done.begin(), done.end());
+    chunk_ranges(C, sym, A->h_order, q);
+    C->n_chunks = (int)done.size();
+    C->chunk_data = C->data;
+    ctx->chunk_m = C;
+  }
+  return LAMB_GPU_OK;
+}
+
 // ---- driver -------------------------------------------------------------------------------
 int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double eps, uint32_t flags,
                       lamb_gpu_mult_stats* stats) {
@@ -850,6 +930,10 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
   double tensor_ops = 0.0;
   int64_t dropped = 0;
   MixedPlanes mp;
+  PanelPair pair;
+  pair.ctx = ctx;
+  std::shared_ptr<GroupTab> c_grp;
+  bool panel = false;
   const bool mixed = (flags & LAMB_GPU_MIXED) != 0;
   // LAMB_GPU_MIXED_MMA_SYNC=1 selects the mma.sync digit kernel for every shape.
   const char* force_sync = std::getenv("LAMB_GPU_MIXED_MMA_SYNC");
@@ -899,19 +983,40 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       LAMB_TRY(pack_plane_meta(ctx, A, mp, &a_offk));
       LAMB_TRY(symbolic_phase(ctx, A, B, C, eps, filt_p, false, a_offk, &sym, mp.b_soff));
     } else {
-      LAMB_TRY(pack_offk(ctx, A, true, &a_offk));
+      if (panel_ok(A, B)) {
+        LAMB_TRY(product_groups(ctx, A, B, &c_grp));
+        trace_mark(ctx, "atom groups");
+        // queued before the count kernel: the totals arrive with the counts
+        panel = panel_gain(nullptr, *A->rgrp, *A->cgrp, *c_grp, A->h_row_bs, B->h_col_bs, 0, nullptr) >= kPanelGain;
+        if (panel)
+          LAMB_TRY(panel_index(ctx, &pair, A, true, B, false, A->rgrp, A->cgrp, c_grp, ctx->pin + kPinPanel));
+      }
       sym.chunked_fill = true;
-      LAMB_TRY(symbolic_phase(ctx, A, B, C, eps, filt_p, false, a_offk, &sym));
+      sym.want_bits = panel;
+      LAMB_TRY(symbolic_phase(ctx, A, B, C, eps, filt_p, false, nullptr, &sym));
+      if (c_grp) {
+        C->rgrp = A->rgrp;
+        C->cgrp = c_grp;
+      }
     }
     trace_mark(ctx, "symbolic");
     if (mixed) LAMB_TRY(build_work(ctx, C, sym, A, &work, &work_c, true));
     LAMB_TRY(dalloc(ctx, &c_nrm, std::max<int64_t>(sym.c_nnz, 1)));
     trace_mark(ctx, "work items");
     if (timed) LAMB_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
-    if (mixed)
+    if (mixed) {
       LAMB_TRY(numeric_mixed(ctx, A, B, C, sym, work, work_c, c_nrm, mp));
-    else
-      LAMB_TRY(numeric_chunks(ctx, A, B, C, sym, a_offk, c_nrm));
+    } else {
+      // an infinity or NaN would meet the zero rows of absent blocks: such operands take the stacks
+      panel = panel && sym.finite && sym.c_nnz > 0 &&
+              panel_gain(&pair, *A->rgrp, *A->cgrp, *c_grp, A->h_row_bs, B->h_col_bs, sym.n_ent, ctx->pin + kPinPanel) >=
+                  kPanelGain;
+      if (panel) LAMB_TRY(numeric_panel(ctx, A, C, sym, &pair, eps, filt_r ? c_nrm : nullptr, !timed, &panel));
+      if (!panel) {
+        LAMB_TRY(pack_offk(ctx, A, true, &a_offk));
+        LAMB_TRY(numeric_chunks(ctx, A, B, C, sym, a_offk, c_nrm));
+      }
+    }
     trace_mark(ctx, "numeric");
     if (timed) LAMB_CUDA(ctx, cudaEventRecord(ctx->ev[2], ctx->stream));
     if (filt_r) LAMB_TRY(result_filter(ctx, C, c_nrm, eps));
@@ -943,6 +1048,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
   st.kernel_launches = (int32_t)(ctx->launches - launches0);
   if (timed) {
     LAMB_CUDA(ctx, cudaEventSynchronize(ctx->ev[3]));
+    LAMB_TRY(check_tiles(ctx));
     float t01 = 0, t12 = 0, t03 = 0, t23 = 0, t04 = 0;
     cudaEventElapsedTime(&t01, ctx->ev[0], ctx->ev[1]);
     cudaEventElapsedTime(&t12, ctx->ev[1], ctx->ev[2]);

@@ -48,6 +48,13 @@ struct Symbolic {
   int32_t fill_n_words = 0, fill_na_max = 0, fill_nc_max = 0;
   double fill_eps = 0.0;
   size_t fill_smem = 0;
+  // set want_bits before symbolic_phase: C's pattern as a bitmap (32 columns a
+  // word) and every row's blocks before each word
+  bool want_bits = false;
+  uint32_t* c_bm = nullptr;
+  int32_t* c_pre = nullptr;
+  bool filter_acts = false;  // some product may fall below eps
+  bool finite = false;       // every block norm of both operands is finite
 };
 void free_symbolic(Ctx* ctx, Symbolic& s);
 
