@@ -117,7 +117,8 @@ struct Ctx {
 // Words of the pinned buffer.
 constexpr int kPinCount = 0;    // what the symbolic count leaves (CountStat, 5 words)
 constexpr int kPinPanel = 5;    // panel totals
-constexpr int kPinTileErr = 8;  // tile_err after the last panel product
+constexpr int kPinOdd = 8;       // non-finite values met while packing (the adjoint's two products)
+constexpr int kPinTileErr = 10;  // tile_err after the last panel product
 constexpr int kPinWords = 64;
 // The smallest and the largest of a matrix's block norms, as bit patterns that
 // an atomic maximum can collect (norms are >= 0 or NaN; a NaN is the largest).

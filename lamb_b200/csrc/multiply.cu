@@ -859,28 +859,6 @@ static int32_t numeric_chunks(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C
 }
 
 // ---- FP64 numeric phase on group tiles -------------------------------------------------
-// Whether the panel kernel may be considered: its block sizes, and about half a
-// million block products (below that the launches that prepare the panels, some
-// 60 us, cost more than the stacks: 48 atoms of 0 to 3 rows, 53,000 products,
-// 625 us a call with stacks, 690 us with panels; 64 waters, 1.6 million, even).
-static bool panel_ok(const DevMatrix* A, const DevMatrix* B) {
-  return A->n_cols > 0 && (double)A->nnz * B->nnz >= (double)(1 << 19) * A->n_cols &&
-         panel_shapes_ok(A->h_row_bs, A->h_col_bs, B->h_col_bs);
-}
-
-// Groups of C's columns: A's when B lives on the same atoms (both then describe
-// the same runs), B's own otherwise.
-static int32_t product_groups(Ctx* ctx, DevMatrix* A, DevMatrix* B, std::shared_ptr<GroupTab>* cols) {
-  LAMB_TRY(ensure_groups(ctx, A));
-  if (A->h_row_bs == A->h_col_bs && B->h_row_bs == A->h_row_bs && B->h_col_bs == A->h_row_bs) {
-    *cols = A->rgrp;
-    return LAMB_GPU_OK;
-  }
-  LAMB_TRY(ensure_groups(ctx, B));
-  *cols = B->cgrp;
-  return LAMB_GPU_OK;
-}
-
 // The tile kernel, in kMinChunks launches when a download may overlap them.
 // *ran = false (nothing done) when the panels do not fit.
 static int32_t numeric_panel(Ctx* ctx, DevMatrix* A, DevMatrix* C, const Symbolic& sym, PanelPair* pair, double eps,
@@ -983,7 +961,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       LAMB_TRY(pack_plane_meta(ctx, A, mp, &a_offk));
       LAMB_TRY(symbolic_phase(ctx, A, B, C, eps, filt_p, false, a_offk, &sym, mp.b_soff));
     } else {
-      if (panel_ok(A, B)) {
+      if (panel_worth(A, B)) {
         LAMB_TRY(product_groups(ctx, A, B, &c_grp));
         trace_mark(ctx, "atom groups");
         // queued before the count kernel: the totals arrive with the counts

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_panel_pack(const __grid_con
   __shared__ long long blk_all[kPackWarps][kGrpAtoms * kGrpAtoms];
   const int lane = threadIdx.x & 31;
   long long* blk = blk_all[threadIdx.x >> 5];
+  bool odd = false;  // an infinity or a NaN among the values
   for (int64_t sb = global_warp(); sb < s.n_sb; sb += grid_warps()) {
     const int g = s.sbg[sb], kg = s.kc[sb];
     const int o0 = s.o_first[g], no = s.o_first[g + 1] - o0;
@@ -252,9 +253,11 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_panel_pack(const __grid_con
         if (o >= 0) v = __ldg(s.data + o + (s.rows_out ? ye + xe * yb : xe + ye * xb));
       }
       if (lane < kW) dst[kk * kW + lane] = v;
+      odd |= !(fabs(v) < INFINITY);
     }
     __syncwarp();
   }
+  if (odd) p.totals[3] = 1;
 }
 
 // ---- macro tiles ------------------------------------------------------------------------
@@ -840,7 +843,8 @@ int32_t make_groups(Ctx* ctx, std::vector<int32_t> first, const std::vector<int8
   uint16_t* hg = reinterpret_cast<uint16_t*>(h.data() + words);
   int32_t *hf = h.data(), *ho = hf + n + 1, *hr = ho + n, *hw = hr + n, *hm = hw + n, *ha = hm + na;
   std::vector<int32_t> pos(na);
-  if ((int)order.size() == na)
+  t->ordered = (int)order.size() == na;
+  if (t->ordered)
     for (int w = 0; w < na; ++w) pos[order[w]] = w;
   else
     std::iota(pos.begin(), pos.end(), 0);
@@ -911,6 +915,10 @@ GroupTab::~GroupTab() {
 }
 
 int32_t ensure_groups(Ctx* ctx, DevMatrix* m) {
+  if (m->rgrp && !m->rgrp->ordered && !m->h_order.empty()) {  // made before the order was known
+    m->rgrp.reset();
+    m->cgrp.reset();
+  }
   if (m->rgrp && m->cgrp) return LAMB_GPU_OK;
   std::vector<int32_t> cnt, both;
   if (!m->cgrp) {
@@ -946,11 +954,28 @@ double panel_gain(const PanelPair* p, const GroupTab& rows, const GroupTab& inne
   return per_pair * mean_slabs(row_bs) * mean_slabs(col_bs);
 }
 
-bool panel_shapes_ok(const std::vector<int8_t>& rows, const std::vector<int8_t>& inner, const std::vector<int8_t>& cols) {
+static bool panel_shapes_ok(const std::vector<int8_t>& rows, const std::vector<int8_t>& inner,
+                            const std::vector<int8_t>& cols) {
   // 51,200 columns of single-atom groups are what the masks of one super row hold in shared memory
   return !rows.empty() && !cols.empty() && !inner.empty() && max_block(rows) <= kGrpRows &&
          max_block(inner) <= kGrpRows && max_block(cols) <= kGrpRows && cols.size() <= 51200 && rows.size() <= 262144 &&
          inner.size() <= 65536;
+}
+
+bool panel_worth(const DevMatrix* A, const DevMatrix* B) {
+  return A->n_cols > 0 && (double)A->nnz * B->nnz >= (double)(1 << 19) * A->n_cols &&
+         panel_shapes_ok(A->h_row_bs, A->h_col_bs, B->h_col_bs);
+}
+
+int32_t product_groups(Ctx* ctx, DevMatrix* A, DevMatrix* B, std::shared_ptr<GroupTab>* cols) {
+  LAMB_TRY(ensure_groups(ctx, A));
+  if (A->h_row_bs == A->h_col_bs && B->h_row_bs == A->h_row_bs && B->h_col_bs == A->h_row_bs) {
+    *cols = A->rgrp;
+    return LAMB_GPU_OK;
+  }
+  LAMB_TRY(ensure_groups(ctx, B));
+  *cols = B->cgrp;
+  return LAMB_GPU_OK;
 }
 
 PanelPair::~PanelPair() {
@@ -981,6 +1006,7 @@ PairArgs pair_args(const PanelPair& p) {
   r.kstride = p.kstride;
   r.nk_max = p.a.in->max_atoms;
   r.n_in = p.a.in->n;
+  r.totals = p.totals;
   return r;
 }
 
@@ -994,7 +1020,7 @@ int32_t panel_index(Ctx* ctx, PanelPair* p, const DevMatrix* ma, bool a_rows_out
   p->a.m = ma; p->a.rows_out = a_rows_out; p->a.out = out_a.get();
   p->b.m = mb; p->b.rows_out = b_rows_out; p->b.out = out_b.get();
   p->kstride = std::max((in->max_rows + 3) & ~3, 4);
-  int64_t* d_tot = nullptr;
+  p->totals = nullptr;
   for (PanelSide* s : {&p->a, &p->b}) {
     s->in = in.get();
     s->words = (in->n + 31) / 32;
@@ -1002,15 +1028,14 @@ int32_t panel_index(Ctx* ctx, PanelPair* p, const DevMatrix* ma, bool a_rows_out
     char* d = nullptr;
     LAMB_TRY(dalloc(ctx, &d, 4 * (in->n + 2 * nw + n1) + 64));
     s->buf = d;
-    if (!d_tot) d_tot = reinterpret_cast<int64_t*>(d);
+    if (!p->totals) p->totals = reinterpret_cast<int64_t*>(d);
     s->hist = reinterpret_cast<int32_t*>(d + 64);
     s->bm = reinterpret_cast<uint32_t*>(s->hist + in->n);
     s->pre = reinterpret_cast<int32_t*>(s->bm + nw);
     s->ptr = s->pre + nw;
-    LAMB_CUDA(ctx, cudaMemsetAsync(s->hist, 0, sizeof(uint32_t) * (in->n + nw), ctx->stream));
+    LAMB_CUDA(ctx, cudaMemsetAsync(d, 0, 64 + sizeof(uint32_t) * (in->n + nw), ctx->stream));
   }
   PairArgs r = pair_args(*p);
-  r.totals = d_tot;
   const int rows = std::max(ma->n_rows, mb->n_rows), outs = std::max(p->a.out->n, p->b.out->n);
   k_panel_bits<<<dim3(grid_for(32ll * rows), 2), kThreads, 0, ctx->stream>>>(r);
   LAMB_LAUNCHED(ctx);
@@ -1018,7 +1043,7 @@ int32_t panel_index(Ctx* ctx, PanelPair* p, const DevMatrix* ma, bool a_rows_out
   LAMB_LAUNCHED(ctx);
   k_panel_scan<<<2, 1024, 0, ctx->stream>>>(r);
   LAMB_LAUNCHED(ctx);
-  LAMB_CUDA(ctx, cudaMemcpyAsync(totals, d_tot, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  LAMB_CUDA(ctx, cudaMemcpyAsync(totals, p->totals, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
   return LAMB_GPU_OK;
 }
 
@@ -1057,6 +1082,45 @@ int32_t panel_pack(Ctx* ctx, PanelPair* p, const int64_t* totals, bool filt, boo
     k_panel_pack<false><<<g, 32 * kPackWarps, 0, ctx->stream>>>(r);
   LAMB_LAUNCHED(ctx);
   *ok = true;
+  return LAMB_GPU_OK;
+}
+
+// Bitmap of a block pattern and every row's blocks before each word, one warp per row.
+__global__ void k_pattern_bits(int32_t n_rows, int32_t n_words, const int64_t* __restrict__ row_p,
+                               const int32_t* __restrict__ col, uint32_t* __restrict__ bm, int32_t* __restrict__ pre) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t r = global_warp(); r < n_rows; r += grid_warps()) {
+    const int64_t b0 = row_p[r], b1 = row_p[r + 1];
+    uint32_t* w = bm + r * n_words;
+    int32_t* q = pre + r * n_words;
+    int64_t b = b0;  // first block of the words to come
+    for (int w0 = 0; w0 < n_words; w0 += 32) {
+      uint32_t mine = 0;
+      const int64_t end = lower_col(col, b, b1, 32 * (w0 + 32));
+      for (int64_t x = b; x < end; x += 32) {
+        // a block's column names its word among the 32 of this step
+        const int c = x + lane < end ? col[x + lane] : -1;
+        for (int s = 0; s < 32; ++s) {
+          const int cs = __shfl_sync(0xffffffffu, c, s);
+          if (cs >= 0 && (cs >> 5) == w0 + lane) mine |= 1u << (cs & 31);
+        }
+      }
+      const int n = __popc(mine), incl = warp_incl_scan(n, lane);
+      if (w0 + lane < n_words) {
+        w[w0 + lane] = mine;
+        q[w0 + lane] = (int32_t)(b - b0) + incl - n;
+      }
+      b = end;
+    }
+  }
+}
+
+int32_t panel_pattern(Ctx* ctx, const DevMatrix* Z, uint32_t** bm, int32_t** pre) {
+  const int32_t words = (Z->n_cols + 31) / 32;
+  LAMB_TRY(dalloc(ctx, bm, (int64_t)Z->n_rows * words));
+  LAMB_TRY(dalloc(ctx, pre, (int64_t)Z->n_rows * words));
+  k_pattern_bits<<<grid_for(32ll * Z->n_rows), kThreads, 0, ctx->stream>>>(Z->n_rows, words, Z->row_p, Z->col, *bm, *pre);
+  LAMB_LAUNCHED(ctx);
   return LAMB_GPU_OK;
 }
 

@@ -13,6 +13,7 @@ struct GroupTab {
   Ctx* ctx = nullptr;
   int32_t n = 0, n_atoms = 0;
   int32_t max_rows = 0, max_atoms = 0;  // of any group
+  bool ordered = false;                 // ranks follow a processing order (otherwise the atoms' own)
   std::vector<int32_t> h_first;         // [n + 1] first atom of every group
   std::vector<int32_t> h_minpos;        // [n] by rank: smallest processing position of the group's atoms
   // one device buffer holding, in this order:
@@ -57,11 +58,21 @@ struct PanelPair {
   PanelSide a, b;
   std::shared_ptr<GroupTab> keep[3];
   int32_t kstride = 0;  // panel rows of a superblock (a multiple of four)
+  // device: superblocks of a and b, superblock pairs, and (after the packing)
+  // whether a value is infinite or NaN
+  int64_t* totals = nullptr;
   ~PanelPair();
 };
 
-// Shape limits of the panel kernel for out-groups of x's rows / columns.
-bool panel_shapes_ok(const std::vector<int8_t>& rows, const std::vector<int8_t>& inner, const std::vector<int8_t>& cols);
+// Whether the panel kernel may be considered for A.B (or its adjoint): its block
+// sizes, and about half a million block products (below that the launches that
+// prepare the panels, some 60 us, cost more than the stacks: 48 atoms of 0 to 3
+// rows, 53,000 products, 625 us a call with stacks, 690 us with panels; 64
+// waters, 1.6 million, even).
+bool panel_worth(const DevMatrix* A, const DevMatrix* B);
+// Groups of A.B's columns (those of its rows and inner atoms are A's): A's when
+// B lives on the same atoms (both then describe the same runs), B's own otherwise.
+int32_t product_groups(Ctx* ctx, DevMatrix* A, DevMatrix* B, std::shared_ptr<GroupTab>* cols);
 // What the panel kernel has to gain on the stack kernel: block products per
 // superblock pair times the stack kernel's 16 x 16 slabs per product.  Measured
 // (ms, stacks -> panels): 1 (atoms of 13 rows that form no groups) 3.1 -> 6.4,
@@ -81,6 +92,8 @@ int32_t panel_index(Ctx* ctx, PanelPair* p, const DevMatrix* ma, bool a_rows_out
 // Panels of both operands (after the totals have arrived); filt: with block
 // norms.  *ok = false, and nothing queued, when they are too large.
 int32_t panel_pack(Ctx* ctx, PanelPair* p, const int64_t* totals, bool filt, bool* ok);
+// Pattern bitmap of Z for panel_tiles (freed by the caller).
+int32_t panel_pattern(Ctx* ctx, const DevMatrix* Z, uint32_t** bm, int32_t** pre);
 // C := product on C's pattern (row_p, off and data set; c_bm / c_pre: the
 // pattern's bitmap over the columns, 32 to a word, and the row's blocks before
 // every word).  c_nrm may be null.  `chunks` launches; done_pos gets the rows

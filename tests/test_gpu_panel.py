@@ -174,3 +174,47 @@ def test_chunked_download_after_async(gpu_ctx):
         assert np.array_equal(s1.extents, s2.extents) and np.array_equal(s1.data, s2.data)
     for x in (db, da):
         x.destroy()
+
+
+@pytest.mark.parametrize("sizes", ["molecule", "edge", "empty", "full", "beyond"])
+@pytest.mark.parametrize("bad", [None, np.inf])
+def test_adjoint(gpu_ctx, sizes, bad):
+    """Both masked products over group tiles; a dC on a pattern that is not
+    A.B's, and with an infinity (then only its own products see it)."""
+    rng = np.random.default_rng(len(sizes))
+    n = 110
+    bs = np.resize(np.array(SIZES[sizes]), n)
+    base = rng.random((3, n // 3 + 1, n // 3 + 1)) < 0.7
+    pa, pb, pc = (np.kron(x, np.ones((3, 3), bool))[:n, :n] & (rng.random((n, n)) < 0.95) for x in base)
+    a, b, dc = (_matrix(rng, bs, bs, p, cut=(40, 40)) for p in (pa, pb, pc))
+    if bad is not None:
+        dc.sectors[1].data[0] = bad
+    da, db, ddc = (gpu_ctx.upload(x) for x in (a, b, dc))
+    ga, gb = gpu_ctx.create_like(da), gpu_ctx.create_like(db)
+    gpu_ctx.adjoint(da, db, ddc, ga, gb)
+    A, B, D = a.to_dense(), b.to_dense(), dc.to_dense()
+    with np.errstate(invalid="ignore"):
+        if bad is None:
+            want = {"a": D @ B.T, "b": A.T @ D}
+        else:  # block by block, so that 0 * inf does not spread
+            off = np.concatenate([[0], np.cumsum(bs)])
+            want = {"a": np.zeros_like(A), "b": np.zeros_like(B)}
+            for i in range(n):
+                for k in range(n):
+                    I, K = slice(off[i], off[i + 1]), slice(off[k], off[k + 1])
+                    for j in np.nonzero(pc[i] & pb[k])[0]:
+                        J = slice(off[j], off[j + 1])
+                        want["a"][I, K] += D[I, J] @ B[K, J].T
+                    for j in np.nonzero(pa[:, i] & pc[:, k])[0]:
+                        J = slice(off[j], off[j + 1])
+                        want["b"][I, K] += A[J, I].T @ D[J, K]
+    for got, ref, p in ((ga.download(), want["a"], pa), (gb.download(), want["b"], pb)):
+        mask = np.repeat(np.repeat(p, bs, 0), bs, 1)
+        g = got.to_dense()
+        assert [s.n_blks for s in got.sectors] == [int(p[r, c].sum()) for r in (slice(0, 40), slice(40, n))
+                                                  for c in (slice(0, 40), slice(40, n))]
+        fin = np.isfinite(ref) & mask
+        assert np.array_equal(np.isfinite(g) & mask, fin)
+        assert np.linalg.norm(g[fin] - ref[fin]) <= 1e-13 * np.linalg.norm(ref[fin])
+    for x in (gb, ga, ddc, db, da):
+        x.destroy()
