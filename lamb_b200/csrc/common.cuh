@@ -288,14 +288,6 @@ struct Walk {
 __device__ __forceinline__ int64_t global_warp() { return ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
 __device__ __forceinline__ int64_t grid_warps() { return ((int64_t)gridDim.x * blockDim.x) >> 5; }
 
-// Fixed-order block norm: sequential fma over the block in storage order.
-// The CPU oracle uses the same expression, so the filter decisions agree bit for bit.
-__device__ __forceinline__ double block_norm_seq(const double* __restrict__ x, int64_t n) {
-  double s = 0.0;
-  for (int64_t e = 0; e < n; ++e) s = __fma_rn(x[e], x[e], s);
-  return __dsqrt_rn(s);
-}
-
 constexpr int kThreads = 256;
 // Counts a launch of one of this library's kernels and checks it.
 #define LAMB_LAUNCHED(ctx) do { ++(ctx)->launches; LAMB_CUDA((ctx), cudaGetLastError()); } while (0)

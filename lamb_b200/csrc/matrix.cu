@@ -230,21 +230,54 @@ int32_t max_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out) {
 }
 
 // ---- block norms -----------------------------------------------------------------------
-// One warp per block row; each lane sums whole blocks sequentially (fixed order).
-__global__ void k_block_norms(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
-                              const int64_t* __restrict__ off, const int8_t* __restrict__ row_bs,
-                              const int8_t* __restrict__ col_bs, const double* __restrict__ data,
-                              double* __restrict__ norms, unsigned long long* __restrict__ range) {
+// One lane per block sums its elements one after the other (the order that
+// decides the filters bit for bit).  A warp brings 32 elements of each of its 32
+// blocks into shared memory at a time, coalesced, so that a lane's chain waits
+// for shared memory only: reading its own block straight from memory a lane's
+// every load touched a sector of its own (144 dense rows: 106 us, now 9 us).
+constexpr int kNormWarps = 4;
+constexpr int kNormStride = 33;  // padded: the lanes of a warp walk distinct banks
+
+__global__ void __launch_bounds__(32 * kNormWarps) k_block_norms(
+    int32_t n_rows, int64_t nnz, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
+    const int64_t* __restrict__ off, const int8_t* __restrict__ row_bs, const int8_t* __restrict__ col_bs,
+    const double* __restrict__ data, double* __restrict__ norms, unsigned long long* __restrict__ range) {
+  __shared__ double stage[kNormWarps][32 * kNormStride];
+  double* st = stage[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   // norms are >= 0 or NaN: their bit patterns order like the values, any NaN above infinity
   unsigned long long lo = 0ull, hi = 0ull;  // largest complement of a pattern, largest pattern
-  for (int64_t r = warp; r < n_rows; r += nwarps) {
-    const int bi = row_bs[r];
-    for (int64_t b = row_p[r] + lane; b < row_p[r + 1]; b += 32) {
-      const int64_t n = (int64_t)bi * col_bs[col[b]];
-      const double v = block_norm_seq(data + off[b], n);
+  for (int64_t w = global_warp(); w * 32 < nnz; w += grid_warps()) {
+    const int64_t b = w * 32 + lane;
+    int n = 0;
+    long long o = 0;
+    if (b < nnz) {
+      int64_t r0 = 0, r1 = n_rows;  // the row r0 with row_p[r0] <= b < row_p[r0 + 1]
+      while (r1 - r0 > 1) {
+        const int64_t mid = (r0 + r1) >> 1;
+        if (row_p[mid] <= b) r0 = mid; else r1 = mid;
+      }
+      n = (int)row_bs[r0] * col_bs[col[b]];
+      o = off[b];
+    }
+    const int n_max = __reduce_max_sync(0xffffffffu, n);
+    double s = 0.0;
+    for (int e0 = 0; e0 < n_max; e0 += 32) {
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i) {
+        const int ni = __shfl_sync(0xffffffffu, n, i);
+        const long long oi = __shfl_sync(0xffffffffu, o, i);
+        if (e0 + lane < ni) st[i * kNormStride + lane] = __ldg(data + oi + e0 + lane);
+      }
+      __syncwarp();
+      const int m = min(32, n - e0);
+      const double* x = st + lane * kNormStride;
+#pragma unroll 4
+      for (int e = 0; e < m; ++e) s = __fma_rn(x[e], x[e], s);
+      __syncwarp();
+    }
+    if (b < nnz) {
+      const double v = __dsqrt_rn(s);
       norms[b] = v;
       const unsigned long long u = (unsigned long long)__double_as_longlong(v);
       lo = max(lo, ~u);
@@ -268,8 +301,8 @@ int32_t ensure_norms(Ctx* ctx, DevMatrix* m) {
   unsigned long long* range = reinterpret_cast<unsigned long long*>(m->norms + m->nnz);
   LAMB_CUDA(ctx, cudaMemsetAsync(range, 0, 2 * sizeof(*range), ctx->stream));
   if (m->nnz > 0) {
-    k_block_norms<<<grid_for((int64_t)m->n_rows * 32), kThreads, 0, ctx->stream>>>(
-        m->n_rows, m->row_p, m->col, m->off, m->row_bs, m->col_bs, m->data, m->norms, range);
+    k_block_norms<<<grid_for(m->nnz, 32 * kNormWarps, 148 * 6), 32 * kNormWarps, 0, ctx->stream>>>(
+        m->n_rows, m->nnz, m->row_p, m->col, m->off, m->row_bs, m->col_bs, m->data, m->norms, range);
     LAMB_LAUNCHED(ctx);
   }
   m->norms_valid = true;

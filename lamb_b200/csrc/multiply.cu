@@ -42,6 +42,10 @@ int32_t check_compatible(Ctx* ctx, const DevMatrix* A, const DevMatrix* B) {
 // One CTA per C block row.  A bitmap over C's block columns marks the columns
 // reached by surviving products A_ik.B_kj (|A_ik|*|B_kj| >= eps).
 constexpr int kSymThreads = 256;
+// Matrices of fewer rows than this (four per SM) run the count with 1,024
+// threads a row: with 256 the eight warps of a row walk a dense row's chains of
+// dependent loads one after the other (288 dense rows: 85 us, now 32 us).
+constexpr int kSymFewRows = 148 * 4;
 
 // No product falls below eps when the smallest norms of A and B multiply to
 // at least eps (fl(x*y) is monotone in x and y); any NaN norm keeps the test.
@@ -55,6 +59,7 @@ __host__ __device__ inline bool filter_acts(const NormRange& a, const NormRange&
   return !finite_norms(a) || !finite_norms(b) || !(bits_to_double(~a.not_min) * bits_to_double(~b.not_min) >= eps);
 }
 // What the host needs of the count kernel beside the rows' counts.
+constexpr int64_t kPatternBitsMax = 2ll << 30;  // bytes of the pattern bitmaps that may be kept
 struct CountStat {
   NormRange a, b;
   unsigned long long max_a_len;
@@ -65,26 +70,29 @@ struct CountStat {
 // 1.4 ms slower at 6,144 waters while the count kernel gains 0.8 ms.
 __device__ __forceinline__ bool keep_norms(double na, double nb, double eps) { return !(na * nb < eps); }
 
-__global__ void __launch_bounds__(kSymThreads) k_sym_count(
+// The bitmaps are kept (g_bm) for the pattern when there is room.
+template <int T>
+__global__ void __launch_bounds__(T) k_sym_count(
     int32_t n_rows, const int64_t* __restrict__ a_row_p, const int32_t* __restrict__ a_col,
     const double* __restrict__ a_nrm, const int64_t* __restrict__ b_row_p, const int32_t* __restrict__ b_col,
     const double* __restrict__ b_nrm, const int8_t* __restrict__ row_bs, const int8_t* __restrict__ k_bs,
     const int8_t* __restrict__ col_bs, double eps, int want_filt, const NormRange* __restrict__ range_a,
-    const NormRange* __restrict__ range_b, int32_t n_words, int64_t* __restrict__ c_cnt, int64_t* __restrict__ s_cnt, int64_t* __restrict__ p_cnt, double* __restrict__ row_flops,
-    CountStat* __restrict__ stat) {
+    const NormRange* __restrict__ range_b, int32_t n_words, int64_t* __restrict__ c_cnt, int64_t* __restrict__ s_cnt,
+    int64_t* __restrict__ p_cnt, double* __restrict__ row_flops, CountStat* __restrict__ stat,
+    uint32_t* __restrict__ g_bm) {
   extern __shared__ uint32_t bm[];
-  typedef cub::BlockReduce<int64_t, kSymThreads> RI;
-  typedef cub::BlockReduce<double, kSymThreads> RD;
+  typedef cub::BlockReduce<int64_t, T> RI;
+  typedef cub::BlockReduce<double, T> RD;
   __shared__ typename RI::TempStorage ti;
   __shared__ typename RD::TempStorage td;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kSymThreads / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = T / 32;
   const bool filt = want_filt && filter_acts(*range_a, *range_b, eps);
   if (blockIdx.x == 0 && tid == 0) {
     stat->a = *range_a;
     stat->b = *range_b;
   }
   for (int64_t i = blockIdx.x; i < n_rows; i += gridDim.x) {
-    for (int w = tid; w < n_words; w += kSymThreads) bm[w] = 0u;
+    for (int w = tid; w < n_words; w += T) bm[w] = 0u;
     __syncthreads();
     int64_t kept = 0, pairs = 0;
     double fl = 0.0;
@@ -98,14 +106,17 @@ __global__ void __launch_bounds__(kSymThreads) k_sym_count(
         ++pairs;
         if (filt && !keep_norms(na, b_nrm[bb], eps)) continue;
         const int j = b_col[bb];
-        atomicOr(&bm[j >> 5], 1u << (j & 31));
+        if (!((bm[j >> 5] >> (j & 31)) & 1u)) atomicOr(&bm[j >> 5], 1u << (j & 31));
         ++kept;
         fl += 2.0 * bi * bk * col_bs[j];
       }
     }
     __syncthreads();
     int64_t pc = 0;
-    for (int w = tid; w < n_words; w += kSymThreads) pc += __popc(bm[w]);
+    for (int w = tid; w < n_words; w += T) {
+      pc += __popc(bm[w]);
+      if (g_bm) g_bm[i * n_words + w] = bm[w];
+    }
     int64_t tot_pc = RI(ti).Sum(pc);
     __syncthreads();
     int64_t tot_kept = RI(ti).Sum(kept);
@@ -151,14 +162,42 @@ __device__ __forceinline__ int bm_rank(const uint32_t* bm, const int* wpre, int 
   return wpre[j >> 5] + __popc(bm[j >> 5] & ((1u << (j & 31)) - 1u));
 }
 
+// C pattern from the count kernel's bitmaps, one warp per row: the blocks before
+// every word (kept for the tile kernel's lookups) and the columns in ascending
+// order.
+__global__ void __launch_bounds__(kSymThreads) k_sym_expand(int32_t n_rows, int32_t n_words,
+                                                            const uint32_t* __restrict__ bm,
+                                                            const int64_t* __restrict__ c_row_p,
+                                                            int32_t* __restrict__ pre, int32_t* __restrict__ c_col) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t i = global_warp(); i < n_rows; i += grid_warps()) {
+    const int64_t c0 = c_row_p[i];
+    int carry = 0;
+    for (int w0 = 0; w0 < n_words; w0 += 32) {
+      const int w = w0 + lane;
+      const uint32_t mine = w < n_words ? bm[i * n_words + w] : 0u;
+      const int n = __popc(mine), incl = warp_incl_scan(n, lane), at = carry + incl - n;
+      if (pre && w < n_words) pre[i * n_words + w] = at;
+      // the 32 words' columns, 32 consecutive blocks at a time
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      for (int s = 0; s < 32; ++s) {
+        const uint32_t word = __shfl_sync(0xffffffffu, mine, s);
+        const int first = __shfl_sync(0xffffffffu, at, s);
+        if ((word >> lane) & 1u) c_col[c0 + first + __popc(word & ((1u << lane) - 1u))] = 32 * (w0 + s) + lane;
+      }
+      carry += total;
+    }
+  }
+}
+
 // C pattern only (no stacks), one CTA per C row: the bitmap of reached
-// columns, then the row's columns in ascending order.  Used by the mixed
-// tensor-core path, which needs no block-product stacks.
+// columns, then the row's columns in ascending order.  For patterns whose
+// bitmaps would take too much memory to keep.
 __global__ void __launch_bounds__(kSymThreads) k_sym_pattern(
     int32_t n_rows, const int64_t* __restrict__ a_row_p, const int32_t* __restrict__ a_col,
     const double* __restrict__ a_nrm, const int64_t* __restrict__ b_row_p, const int32_t* __restrict__ b_col,
     const double* __restrict__ b_nrm, double eps, int32_t n_words, const int64_t* __restrict__ c_row_p,
-    int32_t* __restrict__ c_col, uint32_t* __restrict__ g_bm, int32_t* __restrict__ g_pre) {
+    int32_t* __restrict__ c_col) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t* bm = reinterpret_cast<uint32_t*>(smem_raw);
   int* wpre = reinterpret_cast<int*>(bm + n_words);
@@ -183,10 +222,6 @@ __global__ void __launch_bounds__(kSymThreads) k_sym_pattern(
     for (int w = tid; w < n_words; w += kSymThreads) {
       uint32_t bits = bm[w];
       int p = wpre[w];
-      if (g_bm) {
-        g_bm[i * n_words + w] = bits;
-        g_pre[i * n_words + w] = p;
-      }
       while (bits) {
         const int b = __ffs(bits) - 1;
         bits &= bits - 1u;
@@ -318,10 +353,10 @@ __global__ void __launch_bounds__(kSymThreads) k_sym_fill(
 // Grid of a row-looping symbolic kernel: the CTAs that are resident at once
 // on all SMs (at most one per row).
 template <typename K>
-static int32_t resident_grid(Ctx* ctx, K kern, size_t smem, int32_t n_rows, int* grid) {
+static int32_t resident_grid(Ctx* ctx, K kern, size_t smem, int32_t n_rows, int* grid, int threads = kSymThreads) {
   int sms = 148, per_sm = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  LAMB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSymThreads, smem));
+  LAMB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
   *grid = std::max(1, std::min(n_rows, sms * std::max(per_sm, 1)));
   return LAMB_GPU_OK;
 }
@@ -376,15 +411,20 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
   const size_t smem_count = sizeof(uint32_t) * (size_t)std::max(n_words, 1);
   if (smem_count > 200 * 1024)
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "too many block columns for the symbolic bitmap");
+  const bool keep_bits = (out->pattern_only || out->chunked_fill) && n_rows > 0 &&
+                         4 * (int64_t)n_rows * n_words <= kPatternBitsMax;
+  if (keep_bits) LAMB_TRY(dalloc(ctx, &out->c_bm, (int64_t)n_rows * std::max(n_words, 1)));
   if (n_rows > 0) {
-    auto count_kern = k_sym_count;
+    const bool few = n_rows < kSymFewRows;
+    auto count_kern = few ? k_sym_count<1024> : k_sym_count<kSymThreads>;
     if (smem_count > 48 * 1024)
       LAMB_CUDA(ctx, cudaFuncSetAttribute(count_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
     int grid = 1;
-    LAMB_TRY(resident_grid(ctx, count_kern, smem_count, n_rows, &grid));
-    count_kern<<<grid, kSymThreads, smem_count, ctx->stream>>>(
+    LAMB_TRY(resident_grid(ctx, count_kern, smem_count, n_rows, &grid, few ? 1024 : kSymThreads));
+    count_kern<<<grid, few ? 1024 : kSymThreads, smem_count, ctx->stream>>>(
         n_rows, A->row_p, A->col, A->norms, B->row_p, B->col, B->norms, C->row_bs, B->row_bs, C->col_bs, eps, filt,
-        range(A), range(B), n_words, c_cnt, s_cnt, p_cnt, rfl, d_stat);
+        range(A), range(B), n_words, c_cnt, s_cnt, p_cnt, rfl, d_stat,
+        out->c_bm);
     LAMB_LAUNCHED(ctx);
   }
   unsigned max_na = 0;
@@ -448,19 +488,20 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     if (smem_fill > 220 * 1024)
       return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "C block row too long for the symbolic fill");
   }
-  if (pattern_now && n_rows > 0 && C->nnz > 0) {
+  if (pattern_now && n_rows > 0 && C->nnz > 0 && keep_bits) {
+    if (out->want_bits) LAMB_TRY(dalloc(ctx, &out->c_pre, (int64_t)n_rows * n_words));
+    k_sym_expand<<<grid_for(32ll * n_rows), kSymThreads, 0, ctx->stream>>>(n_rows, n_words, out->c_bm, C->row_p,
+                                                                       out->c_pre, C->col);
+    LAMB_LAUNCHED(ctx);
+    if (!out->want_bits) dfree(ctx, out->c_bm);
+  } else if (pattern_now && n_rows > 0 && C->nnz > 0) {
     const size_t smem_pat = sizeof(uint32_t) * 2 * (size_t)std::max(n_words, 1);
     if (smem_pat > 48 * 1024)
       LAMB_CUDA(ctx, cudaFuncSetAttribute(k_sym_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_pat));
-    if (out->want_bits) {
-      LAMB_TRY(dalloc(ctx, &out->c_bm, (int64_t)n_rows * n_words));
-      LAMB_TRY(dalloc(ctx, &out->c_pre, (int64_t)n_rows * n_words));
-    }
     int pgrid = 1;
     LAMB_TRY(resident_grid(ctx, k_sym_pattern, smem_pat, n_rows, &pgrid));
     k_sym_pattern<<<pgrid, kSymThreads, smem_pat, ctx->stream>>>(n_rows, A->row_p, A->col, A->norms, B->row_p, B->col,
-                                                                B->norms, fill_eps, n_words, C->row_p, C->col,
-                                                                out->c_bm, out->c_pre);
+                                                                B->norms, fill_eps, n_words, C->row_p, C->col);
     LAMB_LAUNCHED(ctx);
   } else if (smem_fill > 220 * 1024) {
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "C block row too long for the symbolic fill");
@@ -986,7 +1027,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       LAMB_TRY(numeric_mixed(ctx, A, B, C, sym, work, work_c, c_nrm, mp));
     } else {
       // an infinity or NaN would meet the zero rows of absent blocks: such operands take the stacks
-      panel = panel && sym.finite && sym.c_nnz > 0 &&
+      panel = panel && sym.finite && sym.c_nnz > 0 && sym.c_pre &&
               panel_gain(&pair, *A->rgrp, *A->cgrp, *c_grp, A->h_row_bs, B->h_col_bs, sym.n_ent, ctx->pin + kPinPanel) >=
                   kPanelGain;
       if (panel) LAMB_TRY(numeric_panel(ctx, A, C, sym, &pair, eps, filt_r ? c_nrm : nullptr, !timed, &panel));

@@ -49,7 +49,7 @@ struct Symbolic {
   double fill_eps = 0.0;
   size_t fill_smem = 0;
   // set want_bits before symbolic_phase: C's pattern as a bitmap (32 columns a
-  // word) and every row's blocks before each word
+  // word) and every row's blocks before each word (none when they would be too large)
   bool want_bits = false;
   uint32_t* c_bm = nullptr;
   int32_t* c_pre = nullptr;

@@ -218,3 +218,20 @@ def test_adjoint(gpu_ctx, sizes, bad):
         assert np.linalg.norm(g[fin] - ref[fin]) <= 1e-13 * np.linalg.norm(ref[fin])
     for x in (gb, ga, ddc, db, da):
         x.destroy()
+
+
+@pytest.mark.parametrize("n", [40, 700])
+@pytest.mark.parametrize("top", [3, 6, 24])
+def test_norms_decide_the_filter(gpu_ctx, n, top):
+    """Block norms over element counts around the 32 that are summed at a time,
+    on few rows and on many (1,024 or 256 threads a row): the product filter at
+    the median of the norm products must skip exactly what the oracle skips."""
+    rng = np.random.default_rng([n, top])
+    bs = rng.integers(0, top + 1, n)
+    p = rng.random((n, n)) < (1.0 if n < 100 else 0.05)
+    a, b = _matrix(rng, bs, bs, p), _matrix(rng, bs, bs, p)
+    norms = np.array([np.linalg.norm(v) for v in block_values(a).values()])
+    norms = norms[norms > 0]
+    eps = float(np.median(rng.choice(norms, 1000) * rng.choice(norms, 1000)))
+    c, ref = _check(gpu_ctx, a, b, eps, oracle.NO_RESULT_FILTER)
+    assert rel_frobenius_error(c, ref) <= TOL
