@@ -16,6 +16,7 @@
 
 #include "common.cuh"
 #include "panel.cuh"
+#include "ptx.cuh"
 
 namespace lamb {
 
@@ -234,16 +235,16 @@ int32_t max_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out) {
 // decides the filters bit for bit).  A warp brings 32 elements of each of its 32
 // blocks into shared memory at a time, coalesced, so that a lane's chain waits
 // for shared memory only: reading its own block straight from memory a lane's
-// every load touched a sector of its own (144 dense rows: 106 us, now 9 us).
-constexpr int kNormWarps = 4;
+// every load touched a sector of its own (144 dense rows: 106 us, now 15 us).
+constexpr int kNormWarps = 2;
 constexpr int kNormStride = 33;  // padded: the lanes of a warp walk distinct banks
 
 __global__ void __launch_bounds__(32 * kNormWarps) k_block_norms(
     int32_t n_rows, int64_t nnz, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
     const int64_t* __restrict__ off, const int8_t* __restrict__ row_bs, const int8_t* __restrict__ col_bs,
     const double* __restrict__ data, double* __restrict__ norms, unsigned long long* __restrict__ range) {
-  __shared__ double stage[kNormWarps][32 * kNormStride];
-  double* st = stage[threadIdx.x >> 5];
+  __shared__ double stage[kNormWarps][2][32 * kNormStride];
+  double(*st)[32 * kNormStride] = stage[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   // norms are >= 0 or NaN: their bit patterns order like the values, any NaN above infinity
   unsigned long long lo = 0ull, hi = 0ull;  // largest complement of a pattern, largest pattern
@@ -262,16 +263,30 @@ __global__ void __launch_bounds__(32 * kNormWarps) k_block_norms(
     }
     const int n_max = __reduce_max_sync(0xffffffffu, n);
     double s = 0.0;
-    for (int e0 = 0; e0 < n_max; e0 += 32) {
-#pragma unroll 8
+    // 32 elements of every block on their way while the previous 32 are summed
+    auto fetch = [&](int e0, double* to) {
+#pragma unroll 4
       for (int i = 0; i < 32; ++i) {
         const int ni = __shfl_sync(0xffffffffu, n, i);
         const long long oi = __shfl_sync(0xffffffffu, o, i);
-        if (e0 + lane < ni) st[i * kNormStride + lane] = __ldg(data + oi + e0 + lane);
+        if (e0 + lane < ni)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(to + i * kNormStride + lane)),
+                       "l"(data + oi + e0 + lane)
+                       : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, st[0]);
+    for (int e0 = 0, k = 0; e0 < n_max; e0 += 32, k ^= 1) {
+      if (e0 + 32 < n_max) {
+        fetch(e0 + 32, st[k ^ 1]);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
       __syncwarp();
       const int m = min(32, n - e0);
-      const double* x = st + lane * kNormStride;
+      const double* x = st[k] + lane * kNormStride;
 #pragma unroll 4
       for (int e = 0; e < m; ++e) s = __fma_rn(x[e], x[e], s);
       __syncwarp();
@@ -301,7 +316,7 @@ int32_t ensure_norms(Ctx* ctx, DevMatrix* m) {
   unsigned long long* range = reinterpret_cast<unsigned long long*>(m->norms + m->nnz);
   LAMB_CUDA(ctx, cudaMemsetAsync(range, 0, 2 * sizeof(*range), ctx->stream));
   if (m->nnz > 0) {
-    k_block_norms<<<grid_for(m->nnz, 32 * kNormWarps, 148 * 6), 32 * kNormWarps, 0, ctx->stream>>>(
+    k_block_norms<<<grid_for(m->nnz, 32 * kNormWarps, 148 * 12), 32 * kNormWarps, 0, ctx->stream>>>(
         m->n_rows, m->nnz, m->row_p, m->col, m->off, m->row_bs, m->col_bs, m->data, m->norms, range);
     LAMB_LAUNCHED(ctx);
   }
