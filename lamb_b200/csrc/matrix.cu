@@ -61,6 +61,20 @@ int32_t scratch_bytes(Ctx* ctx, int slot, size_t bytes, void** p) {
   return LAMB_GPU_OK;
 }
 
+int32_t pinned_bytes(Ctx* ctx, int slot, size_t bytes, void** p) {
+  if (bytes > ctx->stage_bytes[slot]) {
+    LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // copies that still use the old one
+    cudaFreeHost(ctx->stage[slot]);
+    ctx->stage[slot] = nullptr;
+    ctx->stage_bytes[slot] = 0;
+    const size_t want = std::max<size_t>(bytes + bytes / 4, 64 * 1024);
+    LAMB_CUDA(ctx, cudaMallocHost(&ctx->stage[slot], want));
+    ctx->stage_bytes[slot] = want;
+  }
+  *p = ctx->stage[slot];
+  return LAMB_GPU_OK;
+}
+
 void release_scratch(Ctx* ctx) {
   for (int i = 0; i < kScrSlots; ++i) {
     if (ctx->scr[i]) cudaFreeAsync(ctx->scr[i], ctx->stream);
@@ -117,8 +131,8 @@ void touch(DevMatrix* m) {
 
 void free_matrix_buffers(Ctx* ctx, DevMatrix* m) {
   touch(m);
-  dfree(ctx, m->row_bs);
-  dfree(ctx, m->col_bs);
+  m->st.reset();
+  m->row_bs = m->col_bs = nullptr;
   dfree(ctx, m->row_p);
   dfree(ctx, m->col);
   dfree(ctx, m->off);
@@ -157,21 +171,71 @@ void copy_structure(DevMatrix* d, const DevMatrix* r, bool rows_from_rows, const
     d->n_csub = c->n_rsub; d->csub_cnt = c->rsub_cnt; d->csub_base = c->rsub_base; d->h_col_bs = c->h_row_bs;
     d->n_cols = c->n_rows;
   }
+  // the same structure as r's: its device copy serves
+  d->st.reset();
+  if (rows_from_rows && cols_from_cols &&
+      (r == c || (r->n_csub == c->n_csub && r->csub_cnt == c->csub_cnt && r->h_col_bs == c->h_col_bs)))
+    d->st = r->st;
+}
+
+StructTab::~StructTab() {
+  if (buf) cudaFreeAsync(buf, ctx->stream);
 }
 
 int32_t upload_block_sizes(Ctx* ctx, DevMatrix* m) {
-  LAMB_TRY(dalloc(ctx, &m->row_bs, std::max(m->n_rows, 1)));
-  LAMB_TRY(dalloc(ctx, &m->col_bs, std::max(m->n_cols, 1)));
-  if (m->n_rows)
-    LAMB_CUDA(ctx, cudaMemcpyAsync(m->row_bs, m->h_row_bs.data(), m->n_rows, cudaMemcpyHostToDevice, ctx->stream));
-  if (m->n_cols)
-    LAMB_CUDA(ctx, cudaMemcpyAsync(m->col_bs, m->h_col_bs.data(), m->n_cols, cudaMemcpyHostToDevice, ctx->stream));
+  if (!m->st) {
+    auto t = std::make_shared<StructTab>();
+    t->ctx = ctx;
+    const size_t nb = (size_t)(m->n_rsub + 1 + m->n_csub + 1) * sizeof(int32_t);
+    std::vector<char> h(nb + m->n_rows + m->n_cols);
+    int32_t* hb = reinterpret_cast<int32_t*>(h.data());
+    std::copy(m->rsub_base.begin(), m->rsub_base.end(), hb);
+    std::copy(m->csub_base.begin(), m->csub_base.end(), hb + m->n_rsub + 1);
+    std::copy(m->h_row_bs.begin(), m->h_row_bs.end(), reinterpret_cast<int8_t*>(h.data() + nb));
+    std::copy(m->h_col_bs.begin(), m->h_col_bs.end(), reinterpret_cast<int8_t*>(h.data() + nb + m->n_rows));
+    LAMB_TRY(dalloc(ctx, &t->buf, (int64_t)h.size()));
+    LAMB_CUDA(ctx, cudaMemcpyAsync(t->buf, h.data(), h.size(), cudaMemcpyHostToDevice, ctx->stream));
+    t->rbase = reinterpret_cast<int32_t*>(t->buf);
+    t->cbase = t->rbase + m->n_rsub + 1;
+    t->row_bs = reinterpret_cast<int8_t*>(t->buf + nb);
+    t->col_bs = t->row_bs + m->n_rows;
+    m->st = std::move(t);
+  }
+  m->row_bs = m->st->row_bs;
+  m->col_bs = m->st->col_bs;
   return LAMB_GPU_OK;
 }
 
 // ---- scans --------------------------------------------------------------------------
+// Short scans in one launch without temporary storage (cub takes two launches
+// and an allocation): up to 8,192 values, eight rounds of one CTA.
+constexpr int64_t kScanSmall = 8192;
+template <bool INCL>
+__global__ void __launch_bounds__(1024) k_scan_small(const int64_t* in, int64_t* out, int64_t n) {
+  typedef cub::BlockScan<long long, 1024> BS;
+  __shared__ typename BS::TempStorage ts;
+  long long carry = 0;
+  for (int64_t x0 = 0; x0 < n; x0 += 1024) {
+    const int64_t x = x0 + threadIdx.x;
+    const long long v = x < n ? in[x] : 0;
+    long long r, a;
+    if (INCL)
+      BS(ts).InclusiveSum(v, r, a);
+    else
+      BS(ts).ExclusiveSum(v, r, a);
+    __syncthreads();
+    if (x < n) out[x] = carry + r;
+    carry += a;
+  }
+}
+
 int32_t exclusive_scan_i64(Ctx* ctx, const int64_t* in, int64_t* out, int64_t n) {
   if (n <= 0) return LAMB_GPU_OK;
+  if (n <= kScanSmall) {
+    k_scan_small<false><<<1, 1024, 0, ctx->stream>>>(in, out, n);
+    LAMB_LAUNCHED(ctx);
+    return LAMB_GPU_OK;
+  }
   size_t bytes = 0;
   LAMB_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, ctx->stream));
   void* tmp = nullptr;
@@ -184,6 +248,11 @@ int32_t exclusive_scan_i64(Ctx* ctx, const int64_t* in, int64_t* out, int64_t n)
 
 int32_t inclusive_scan_i64(Ctx* ctx, const int64_t* in, int64_t* out, int64_t n) {
   if (n <= 0) return LAMB_GPU_OK;
+  if (n <= kScanSmall) {
+    k_scan_small<true><<<1, 1024, 0, ctx->stream>>>(in, out, n);
+    LAMB_LAUNCHED(ctx);
+    return LAMB_GPU_OK;
+  }
   size_t bytes = 0;
   LAMB_CUDA(ctx, cub::DeviceScan::InclusiveSum(nullptr, bytes, in, out, n, ctx->stream));
   void* tmp = nullptr;
@@ -429,20 +498,14 @@ int32_t build_sector_index(Ctx* ctx, const DevMatrix* m, SectorIndex* si) {
   const int64_t n_seq = (int64_t)m->n_rows * S;
   si->h_bcnt.assign(std::max<int64_t>(n_seq, 1), 0);
   if (n_seq == 0 || m->nnz == 0) return LAMB_GPU_OK;
-  int64_t *d_dsz = nullptr, *d_bcnt = nullptr, *d_bpos = nullptr, *d_sbase = nullptr;
-  int32_t *d_rb = nullptr, *d_cb = nullptr;
+  int64_t* d_dsz = nullptr;
+  const int32_t *d_rb = m->st->rbase, *d_cb = m->st->cbase;
   LAMB_TRY(dalloc(ctx, &si->col16, m->nnz));
   LAMB_TRY(dalloc(ctx, &si->ext, 2 * m->nnz));
-  LAMB_TRY(dalloc(ctx, &d_dsz, n_seq));
-  LAMB_TRY(dalloc(ctx, &d_bcnt, n_seq));
-  LAMB_TRY(dalloc(ctx, &d_bpos, n_seq));
-  LAMB_TRY(dalloc(ctx, &d_sbase, (int64_t)m->sec_base.size()));
-  LAMB_TRY(dalloc(ctx, &d_rb, m->n_rsub + 1));
-  LAMB_TRY(dalloc(ctx, &d_cb, S + 1));
-  // the host vectors copied from are members of m: they outlive the copies
+  LAMB_TRY(dalloc(ctx, &d_dsz, 3 * n_seq + (int64_t)m->sec_base.size()));
+  int64_t *d_bcnt = d_dsz + n_seq, *d_bpos = d_bcnt + n_seq, *d_sbase = d_bpos + n_seq;
+  // sec_base is a member of m: it outlives the copy
   LAMB_CUDA(ctx, cudaMemcpyAsync(d_sbase, m->sec_base.data(), sizeof(int64_t) * m->sec_base.size(), cudaMemcpyHostToDevice, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(d_rb, m->rsub_base.data(), sizeof(int32_t) * (m->n_rsub + 1), cudaMemcpyHostToDevice, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(d_cb, m->csub_base.data(), sizeof(int32_t) * (S + 1), cudaMemcpyHostToDevice, ctx->stream));
   k_part_sizes<<<grid_for(32ll * m->n_rows, 256), 256, 0, ctx->stream>>>(m->n_rows, m->n_rsub, S, d_rb, d_cb, m->row_p,
                                                                     m->col, m->row_bs, m->col_bs, nullptr, d_dsz, d_bcnt);
   LAMB_LAUNCHED(ctx);
@@ -452,7 +515,7 @@ int32_t build_sector_index(Ctx* ctx, const DevMatrix* m, SectorIndex* si) {
                                                                       d_sbase, si->col16, si->ext);
   LAMB_LAUNCHED(ctx);
   LAMB_CUDA(ctx, cudaMemcpyAsync(si->h_bcnt.data(), d_bcnt, sizeof(int64_t) * n_seq, cudaMemcpyDeviceToHost, ctx->stream));
-  dfree(ctx, d_dsz); dfree(ctx, d_bcnt); dfree(ctx, d_bpos); dfree(ctx, d_sbase); dfree(ctx, d_rb); dfree(ctx, d_cb);
+  dfree(ctx, d_dsz);
   return LAMB_GPU_OK;
 }
 
@@ -466,10 +529,9 @@ int32_t layout_sector_major(Ctx* ctx, DevMatrix* m, int32_t* row_of, bool by_ord
   const int64_t n_seq = (int64_t)m->n_rows * S;
   // Rank of every row among the rows of its subset, in the processing order
   // (h_order), when the rows' data should follow that order.
-  std::vector<int32_t> h_rank;
-  int32_t* d_rank = nullptr;
+  int32_t *h_rank = nullptr, *d_rank = nullptr;
   if (by_order && (int64_t)m->h_order.size() == m->n_rows && m->n_rows > 0) {
-    h_rank.resize(m->n_rows);
+    LAMB_TRY(pinned(ctx, kPinRank, m->n_rows, &h_rank));
     std::vector<int32_t> next(m->n_rsub, 0), sub_of(m->n_rows);
     for (int a = 0; a < m->n_rsub; ++a)
       for (int r = m->rsub_base[a]; r < m->rsub_base[a + 1]; ++r) sub_of[r] = a;
@@ -480,19 +542,14 @@ int32_t layout_sector_major(Ctx* ctx, DevMatrix* m, int32_t* row_of, bool by_ord
   m->sec_nblk.assign((size_t)m->n_rsub * S, 0);
   if (!m->off) LAMB_TRY(dalloc(ctx, &m->off, std::max<int64_t>(m->nnz, 1)));
   if (n_seq == 0) { m->data_len = 0; return LAMB_GPU_OK; }
-  int32_t *d_rb = nullptr, *d_cb = nullptr;
-  int64_t *dsz = nullptr, *bcnt = nullptr, *dbase = nullptr;
-  LAMB_TRY(dalloc(ctx, &d_rb, m->n_rsub + 1));
-  LAMB_TRY(dalloc(ctx, &d_cb, S + 1));
-  LAMB_TRY(dalloc(ctx, &dsz, n_seq));
-  LAMB_TRY(dalloc(ctx, &bcnt, n_seq));
-  LAMB_TRY(dalloc(ctx, &dbase, n_seq));
-  if (!h_rank.empty()) {
-    LAMB_TRY(dalloc(ctx, &d_rank, m->n_rows));
-    LAMB_CUDA(ctx, cudaMemcpyAsync(d_rank, h_rank.data(), sizeof(int32_t) * m->n_rows, cudaMemcpyHostToDevice, ctx->stream));
+  const int32_t *d_rb = m->st->rbase, *d_cb = m->st->cbase;
+  int64_t* dsz = nullptr;
+  LAMB_TRY(dalloc(ctx, &dsz, 3 * n_seq + (m->n_rows + 1) / 2));
+  int64_t *bcnt = dsz + n_seq, *dbase = bcnt + n_seq;
+  if (h_rank) {
+    d_rank = reinterpret_cast<int32_t*>(dbase + n_seq);
+    LAMB_CUDA(ctx, cudaMemcpyAsync(d_rank, h_rank, sizeof(int32_t) * m->n_rows, cudaMemcpyHostToDevice, ctx->stream));
   }
-  LAMB_CUDA(ctx, cudaMemcpyAsync(d_rb, m->rsub_base.data(), sizeof(int32_t) * (m->n_rsub + 1), cudaMemcpyHostToDevice, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(d_cb, m->csub_base.data(), sizeof(int32_t) * (S + 1), cudaMemcpyHostToDevice, ctx->stream));
   k_part_sizes<<<grid_for(32ll * m->n_rows, 256), 256, 0, ctx->stream>>>(m->n_rows, m->n_rsub, S, d_rb, d_cb, m->row_p,
                                                                     m->col, m->row_bs, m->col_bs, d_rank, dsz, bcnt);
   LAMB_LAUNCHED(ctx);
@@ -501,11 +558,11 @@ int32_t layout_sector_major(Ctx* ctx, DevMatrix* m, int32_t* row_of, bool by_ord
                                                                       m->col, m->row_bs, m->col_bs, dbase, d_rank,
                                                                       m->off, row_of);
   LAMB_LAUNCHED(ctx);
-  std::vector<int64_t> h_dsz(n_seq), h_bcnt(n_seq), h_dbase(n_seq);
-  LAMB_CUDA(ctx, cudaMemcpyAsync(h_dsz.data(), dsz, sizeof(int64_t) * n_seq, cudaMemcpyDeviceToHost, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(h_bcnt.data(), bcnt, sizeof(int64_t) * n_seq, cudaMemcpyDeviceToHost, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(h_dbase.data(), dbase, sizeof(int64_t) * n_seq, cudaMemcpyDeviceToHost, ctx->stream));
+  int64_t* h_dsz = nullptr;
+  LAMB_TRY(pinned(ctx, kPinLayout, 3 * n_seq, &h_dsz));
+  LAMB_CUDA(ctx, cudaMemcpyAsync(h_dsz, dsz, sizeof(int64_t) * 3 * n_seq, cudaMemcpyDeviceToHost, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  const int64_t *h_bcnt = h_dsz + n_seq, *h_dbase = h_bcnt + n_seq;
   for (int a = 0; a < m->n_rsub; ++a)
     for (int n = 0; n < S; ++n) {
       const int64_t cnt = m->rsub_cnt[a];
@@ -518,8 +575,8 @@ int32_t layout_sector_major(Ctx* ctx, DevMatrix* m, int32_t* row_of, bool by_ord
       m->sec_nblk[s] = nb;
     }
   m->data_len = h_dbase[n_seq - 1] + h_dsz[n_seq - 1];
-  if (h_base_out) *h_base_out = std::move(h_dbase);
-  dfree(ctx, d_rb); dfree(ctx, d_cb); dfree(ctx, dsz); dfree(ctx, bcnt); dfree(ctx, dbase); dfree(ctx, d_rank);
+  if (h_base_out) h_base_out->assign(h_dbase, h_dbase + n_seq);
+  dfree(ctx, dsz);
   return LAMB_GPU_OK;
 }
 
@@ -733,6 +790,7 @@ int32_t lamb_gpu_ctx_destroy(lamb_gpu_ctx* c) {
   if (ctx->pend_ev) cudaEventDestroy(ctx->pend_ev);
   if (ctx->pend_h) cudaFreeHost(ctx->pend_h);
   cudaFreeHost(ctx->pin);
+  for (void* x : ctx->stage) cudaFreeHost(x);
   cudaFree(ctx->tile_err);
   cudaStreamDestroy(ctx->stream);
   delete ctx;

@@ -396,12 +396,10 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
   const int32_t n_rows = C->n_rows;
   const int32_t n_words = (C->n_cols + 31) / 32;
   LAMB_TRY(dalloc(ctx, &C->row_p, n_rows + 1));
-  int64_t *c_cnt = nullptr, *s_cnt = nullptr, *p_cnt = nullptr;
-  double* rfl = nullptr;
-  LAMB_TRY(dalloc(ctx, &c_cnt, std::max(n_rows, 1)));
-  LAMB_TRY(dalloc(ctx, &s_cnt, std::max(n_rows, 1)));
-  LAMB_TRY(dalloc(ctx, &p_cnt, std::max(n_rows, 1)));
-  LAMB_TRY(dalloc(ctx, &rfl, std::max(n_rows, 1)));
+  int64_t* c_cnt = nullptr;
+  LAMB_TRY(dalloc(ctx, &c_cnt, 4 * (int64_t)std::max(n_rows, 1)));
+  int64_t *s_cnt = c_cnt + n_rows, *p_cnt = s_cnt + n_rows;
+  double* rfl = reinterpret_cast<double*>(p_cnt + n_rows);
   CountStat* d_stat = nullptr;
   LAMB_TRY(dalloc(ctx, &d_stat, 1));
   LAMB_CUDA(ctx, cudaMemsetAsync(d_stat, 0, sizeof(CountStat), ctx->stream));
@@ -428,14 +426,12 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     LAMB_LAUNCHED(ctx);
   }
   unsigned max_na = 0;
-  std::vector<int64_t> h_s(n_rows), h_p(n_rows);
-  std::vector<double> h_f(n_rows);
-  out->h_row_len.assign(n_rows, 0);
+  int64_t* h_cnt = nullptr;
+  LAMB_TRY(pinned(ctx, kPinCounts, 4 * (int64_t)n_rows, &h_cnt));
+  const int64_t *h_s = h_cnt + n_rows, *h_p = h_s + n_rows;
+  const double* h_f = reinterpret_cast<const double*>(h_p + n_rows);
   if (n_rows) {
-    LAMB_CUDA(ctx, cudaMemcpyAsync(out->h_row_len.data(), c_cnt, sizeof(int64_t) * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
-    LAMB_CUDA(ctx, cudaMemcpyAsync(h_s.data(), s_cnt, sizeof(int64_t) * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
-    LAMB_CUDA(ctx, cudaMemcpyAsync(h_p.data(), p_cnt, sizeof(int64_t) * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
-    LAMB_CUDA(ctx, cudaMemcpyAsync(h_f.data(), rfl, sizeof(double) * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
+    LAMB_CUDA(ctx, cudaMemcpyAsync(h_cnt, c_cnt, sizeof(int64_t) * 4 * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
     LAMB_CUDA(ctx, cudaMemcpyAsync(ctx->pin + kPinCount, d_stat, sizeof(CountStat), cudaMemcpyDeviceToHost, ctx->stream));
     LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
@@ -446,7 +442,11 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     out->finite = finite_norms(h.a) && finite_norms(h.b);
   }
   trace_mark(ctx, "symbolic count");
-  std::vector<int64_t> h_crp(n_rows + 1, 0), h_srb(n_rows + 1, 0);
+  out->h_row_len.assign(h_cnt, h_cnt + n_rows);
+  int64_t* h_crp = nullptr;
+  LAMB_TRY(pinned(ctx, kPinRows, 2 * ((int64_t)n_rows + 1), &h_crp));
+  int64_t* h_srb = h_crp + n_rows + 1;
+  h_crp[0] = h_srb[0] = 0;
   int64_t max_c = 0, max_s = 0;
   for (int r = 0; r < n_rows; ++r) {
     h_crp[r + 1] = h_crp[r] + out->h_row_len[r];
@@ -462,11 +462,14 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "stack too large");
   C->nnz = out->c_nnz;
   int64_t* s_row_base = nullptr;
-  LAMB_TRY(dalloc(ctx, &s_row_base, n_rows + 1));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(C->row_p, h_crp.data(), sizeof(int64_t) * (n_rows + 1), cudaMemcpyHostToDevice, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(s_row_base, h_srb.data(), sizeof(int64_t) * (n_rows + 1), cudaMemcpyHostToDevice, ctx->stream));
+  LAMB_CUDA(ctx, cudaMemcpyAsync(C->row_p, h_crp, sizeof(int64_t) * (n_rows + 1), cudaMemcpyHostToDevice, ctx->stream));
   LAMB_TRY(dalloc(ctx, &C->col, std::max<int64_t>(C->nnz, 1)));
-  LAMB_TRY(dalloc(ctx, &out->stack_p, C->nnz + 1));
+  if (!pattern_now) {
+    LAMB_TRY(dalloc(ctx, &s_row_base, n_rows + 1));
+    LAMB_CUDA(ctx, cudaMemcpyAsync(s_row_base, h_srb, sizeof(int64_t) * (n_rows + 1), cudaMemcpyHostToDevice, ctx->stream));
+    LAMB_TRY(dalloc(ctx, &out->stack_p, C->nnz + 1));
+    LAMB_CUDA(ctx, cudaMemcpyAsync(out->stack_p + C->nnz, &h_srb[n_rows], sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
+  }
   if (want_ids)
     LAMB_TRY(dalloc(ctx, &out->ids, std::max<int64_t>(out->n_ent, 1)));
   else if (pattern_now)
@@ -475,11 +478,10 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     LAMB_TRY(scratch(ctx, kScrEnt, out->n_ent, &out->ent));
   else
     LAMB_TRY(dalloc(ctx, &out->ent, std::max<int64_t>(out->n_ent, 1)));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(out->stack_p + C->nnz, &h_srb[n_rows], sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
   trace_mark(ctx, "symbolic allocations");
   const size_t smem_fill = sym_fill_smem(std::max(n_words, 1), std::max<int64_t>(max_na, 1), max_c);
   if (out->chunked_fill) {
-    out->h_row_ent = h_s;
+    out->h_row_ent.assign(h_s, h_s + n_rows);
     out->fill_n_words = std::max(n_words, 1);
     out->fill_na_max = (int32_t)std::max<int64_t>(max_na, 1);
     out->fill_nc_max = (int32_t)max_c;
@@ -522,7 +524,7 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     LAMB_LAUNCHED(ctx);
   }
   trace_mark(ctx, "symbolic fill");
-  LAMB_TRY(dalloc(ctx, &out->c_row, std::max<int64_t>(C->nnz, 1)));
+  if (!pattern_now) LAMB_TRY(dalloc(ctx, &out->c_row, std::max<int64_t>(C->nnz, 1)));
   LAMB_TRY(layout_sector_major(ctx, C, out->c_row, true, &out->h_base));
   trace_mark(ctx, "sector layout");
   if (C->data_len >= kMask40) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "C data too large");
@@ -536,7 +538,7 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     LAMB_TRY(dalloc(ctx, &C->data, need));
     C->data_cap = need;
   }
-  dfree(ctx, c_cnt); dfree(ctx, s_cnt); dfree(ctx, p_cnt); dfree(ctx, rfl); dfree(ctx, s_row_base);
+  dfree(ctx, c_cnt); dfree(ctx, s_row_base);
   dfree(ctx, d_stat);
   trace_mark(ctx, "C data allocation");
   return LAMB_GPU_OK;
@@ -690,21 +692,16 @@ int32_t result_filter(Ctx* ctx, DevMatrix* C, const double* c_nrm, double eps) {
     ctx->pend_cap = n_sec;
   }
   if (!ctx->pend_ev) LAMB_CUDA(ctx, cudaEventCreateWithFlags(&ctx->pend_ev, cudaEventDisableTiming));
-  int64_t *row_kept = nullptr, *nrp = nullptr, *noff = nullptr;
+  int64_t *nrp = nullptr, *noff = nullptr;
   unsigned long long* sec_kept = nullptr;
-  int32_t *d_cb = nullptr, *d_rb = nullptr, *ncol = nullptr;
-  LAMB_TRY(dalloc(ctx, &row_kept, (int64_t)C->n_rows + 1));
+  int32_t* ncol = nullptr;
+  const int32_t *d_rb = C->st->rbase, *d_cb = C->st->cbase;
+  LAMB_TRY(dalloc(ctx, &sec_kept, (int64_t)n_sec + C->n_rows + 1));
+  int64_t* row_kept = reinterpret_cast<int64_t*>(sec_kept + n_sec);
   LAMB_TRY(dalloc(ctx, &nrp, (int64_t)C->n_rows + 1));
-  LAMB_TRY(dalloc(ctx, &sec_kept, (int64_t)n_sec));
-  LAMB_TRY(dalloc(ctx, &d_cb, S + 1));
-  LAMB_TRY(dalloc(ctx, &d_rb, C->n_rsub + 1));
   LAMB_TRY(dalloc(ctx, &ncol, C->nnz));
   LAMB_TRY(dalloc(ctx, &noff, C->nnz));
-  // csub_base / rsub_base are members of C: they outlive the copies.
-  LAMB_CUDA(ctx, cudaMemcpyAsync(d_cb, C->csub_base.data(), sizeof(int32_t) * (S + 1), cudaMemcpyHostToDevice, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(d_rb, C->rsub_base.data(), sizeof(int32_t) * (C->n_rsub + 1), cudaMemcpyHostToDevice, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemsetAsync(row_kept, 0, sizeof(int64_t), ctx->stream));
-  LAMB_CUDA(ctx, cudaMemsetAsync(sec_kept, 0, sizeof(unsigned long long) * n_sec, ctx->stream));
+  LAMB_CUDA(ctx, cudaMemsetAsync(sec_kept, 0, sizeof(unsigned long long) * (n_sec + 1), ctx->stream));
   k_keep_counts<<<grid_for(32ll * C->n_rows, 256), 256, 0, ctx->stream>>>(C->n_rows, S, d_cb, d_rb, C->n_rsub, C->row_p,
                                                                     C->col, c_nrm, eps, row_kept, sec_kept);
   LAMB_LAUNCHED(ctx);
@@ -718,7 +715,7 @@ int32_t result_filter(Ctx* ctx, DevMatrix* C, const double* c_nrm, double eps) {
   C->row_p = nrp; C->col = ncol; C->off = noff;
   touch(C);
   C->norms_valid = false;
-  dfree(ctx, row_kept); dfree(ctx, sec_kept); dfree(ctx, d_cb); dfree(ctx, d_rb);
+  dfree(ctx, sec_kept);
   ctx->pend_m = C;
   return LAMB_GPU_OK;
 }
@@ -771,8 +768,9 @@ static void chunk_ranges(DevMatrix* C, const Symbolic& sym, const std::vector<in
 // complete.  Inside a sector, C's data follow the processing order
 // (layout_sector_major by_order), so chunk p's data in sector s is one
 // contiguous range.
-static int32_t numeric_chunks(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, const Symbolic& sym,
+static int32_t numeric_chunks(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, Symbolic& sym,
                               const int64_t* a_offk, double* c_nrm) {
+  if (!sym.stack_p) LAMB_TRY(dalloc(ctx, &sym.stack_p, C->nnz + 1));
   const int mi = max_block(A->h_col_bs);
   const int n = C->n_rows, S = C->n_csub, R = C->n_rsub;
   const size_t n_sec = (size_t)R * S;
@@ -913,7 +911,9 @@ static int32_t numeric_panel(Ctx* ctx, DevMatrix* A, DevMatrix* C, const Symboli
                          (int64_t)sym.h_base.size() == (int64_t)n * C->n_csub;
   std::vector<int32_t> done;
   // the tile kernel skips blocks without elements
-  if (c_nrm) LAMB_CUDA(ctx, cudaMemsetAsync(c_nrm, 0, sizeof(double) * sym.c_nnz, ctx->stream));
+  auto empty = [](const std::vector<int8_t>& v) { return std::find(v.begin(), v.end(), 0) != v.end(); };
+  if (c_nrm && (empty(C->h_row_bs) || empty(C->h_col_bs)))
+    LAMB_CUDA(ctx, cudaMemsetAsync(c_nrm, 0, sizeof(double) * sym.c_nnz, ctx->stream));
   LAMB_TRY(panel_tiles(ctx, *pair, C, sym.c_bm, sym.c_pre, c_nrm, sym.filter_acts, eps, overlap && layout_ok ? kMinChunks : 1, &done));
   if (layout_ok) {
     std::vector<int> q(1, 0);
@@ -1020,7 +1020,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
     }
     trace_mark(ctx, "symbolic");
     if (mixed) LAMB_TRY(build_work(ctx, C, sym, A, &work, &work_c, true));
-    LAMB_TRY(dalloc(ctx, &c_nrm, std::max<int64_t>(sym.c_nnz, 1)));
+    if (mixed || filt_r) LAMB_TRY(dalloc(ctx, &c_nrm, std::max<int64_t>(sym.c_nnz, 1)));
     trace_mark(ctx, "work items");
     if (timed) LAMB_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
     if (mixed) {
@@ -1030,7 +1030,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       panel = panel && sym.finite && sym.c_nnz > 0 && sym.c_pre &&
               panel_gain(&pair, *A->rgrp, *A->cgrp, *c_grp, A->h_row_bs, B->h_col_bs, sym.n_ent, ctx->pin + kPinPanel) >=
                   kPanelGain;
-      if (panel) LAMB_TRY(numeric_panel(ctx, A, C, sym, &pair, eps, filt_r ? c_nrm : nullptr, !timed, &panel));
+      if (panel) LAMB_TRY(numeric_panel(ctx, A, C, sym, &pair, eps, c_nrm, !timed, &panel));
       if (!panel) {
         LAMB_TRY(pack_offk(ctx, A, true, &a_offk));
         LAMB_TRY(numeric_chunks(ctx, A, B, C, sym, a_offk, c_nrm));
