@@ -205,6 +205,7 @@ void move_matrix(Ctx* ctx, DevMatrix* dst, DevMatrix* src) {
   float box[3] = {dst->box[0], dst->box[1], dst->box[2]};
   std::vector<int32_t> ord = dst->h_order;
   std::shared_ptr<GroupTab> rg = dst->rgrp, cg = dst->cgrp;
+  std::shared_ptr<ClusterTab> rk = dst->rclu, ck = dst->cclu;
   free_matrix_buffers(ctx, dst);
   *dst = std::move(*src);
   *src = DevMatrix{};
@@ -215,6 +216,10 @@ void move_matrix(Ctx* ctx, DevMatrix* dst, DevMatrix* src) {
   }
   if (dst->h_order.empty() && (int)ord.size() == dst->n_rows) {
     dst->h_order = ord;
+    if (!dst->rclu && !dst->cclu) {
+      dst->rclu = rk;
+      dst->cclu = ck;
+    }
     if (!dst->rgrp && !dst->cgrp && rg && cg && rg->n_atoms == dst->n_rows && cg->n_atoms == dst->n_cols) {
       dst->rgrp = rg;
       dst->cgrp = cg;
@@ -261,6 +266,8 @@ int32_t copy_impl(Ctx* ctx, const DevMatrix* X, DevMatrix* Y) {
   tmp.h_order = X->h_order;
   tmp.rgrp = X->rgrp;
   tmp.cgrp = X->cgrp;
+  tmp.rclu = X->rclu;
+  tmp.cclu = X->cclu;
   LAMB_TRY(upload_block_sizes(ctx, &tmp));
   LAMB_TRY(dalloc(ctx, &tmp.row_p, tmp.n_rows + 1));
   LAMB_TRY(dalloc(ctx, &tmp.col, std::max<int64_t>(tmp.nnz, 1)));

@@ -20,6 +20,7 @@ namespace lamb {
 inline int32_t make_status(int level, int type) { return level * 100000 + (type + 50000); }
 
 struct GroupTab;
+struct ClusterTab;
 struct Ctx;
 
 // Device copy of a structure (subset bases and block sizes), shared by the
@@ -67,6 +68,10 @@ struct DevMatrix {
   int32_t* order = nullptr;      // device copy of h_order
   // Groups of row and column atoms for the panel products (panel.cuh), empty until needed.
   std::shared_ptr<GroupTab> rgrp, cgrp;
+  // Clusters of the row atoms for the mixed tiles, of tile-row and tile-column
+  // width, empty until needed: a function of the row block sizes, the order
+  // and the coordinates alone.
+  std::shared_ptr<ClusterTab> rclu, cclu;
   // Result of a multiply computed in row chunks: the data of chunk p in
   // sector s is [chunk_rng[2*(p*S_all+s)], chunk_rng[2*(p*S_all+s)+1]) relative
   // to the sector's base; chunk p is complete when the context's chunk_ev[p]
@@ -142,6 +147,7 @@ constexpr int kPinCount = 0;    // what the symbolic count leaves (CountStat, 5 
 constexpr int kPinPanel = 5;    // panel totals
 constexpr int kPinOdd = 8;       // non-finite values met while packing (the adjoint's two products)
 constexpr int kPinTileErr = 10;  // tile_err after the last panel product
+constexpr int kPinTc = 16;       // sizes, statistics and error code of the mixed tiles (8 words)
 constexpr int kPinWords = 64;
 // The smallest and the largest of a matrix's block norms, as bit patterns that
 // an atomic maximum can collect (norms are >= 0 or NaN; a NaN is the largest).

@@ -141,6 +141,8 @@ void free_matrix_buffers(Ctx* ctx, DevMatrix* m) {
   dfree(ctx, m->norms);
   dfree(ctx, m->order);
   m->h_order.clear();
+  m->rclu.reset();
+  m->cclu.reset();
   m->rgrp.reset();
   m->cgrp.reset();
   m->norms_valid = false;
@@ -676,6 +678,8 @@ int32_t inherit_row_locality(Ctx* ctx, DevMatrix* dst, const DevMatrix* src) {
   dst->h_pos = src->h_pos;
   memcpy(dst->box, src->box, sizeof(dst->box));
   dst->h_order = src->h_order;
+  dst->rclu = src->rclu;
+  dst->cclu = src->cclu;
   dfree(ctx, dst->order);
   return LAMB_GPU_OK;
 }
@@ -966,6 +970,8 @@ int32_t lamb_gpu_matrix_set_positions(lamb_gpu_ctx* c, lamb_gpu_matrix h, const 
   dfree(ctx, m->order);
   m->rgrp.reset();  // the groups' ranks follow the order
   m->cgrp.reset();
+  m->rclu.reset();
+  m->cclu.reset();
   return LAMB_GPU_OK;
 }
 

@@ -17,9 +17,9 @@
 // Pairs with p + q >= S are dropped (weight below 127^-2 254^-S).
 //
 // Tiles.  Block rows are too small for tcgen05 (M = 128), so the multiply is
-// done on spatial clusters: row atoms (in the row processing order, a Morton
-// curve over the atoms' coordinates) are cut into clusters of at most 128
-// rows, column atoms into clusters of at most 64 columns.  A cluster pair
+// done on spatial clusters: row atoms (nearby ones, k_tc_pool, or without
+// coordinates runs of the row processing order) form clusters of at most 128
+// rows, column atoms clusters of at most 64 columns.  A cluster pair
 // (I, J) holding at least one C block is one tile; its inner dimension is the
 // concatenation of every inner atom k that couples to both clusters (some
 // A_ik with i in I and some B_kj with j in J), so only M and N are padded.
@@ -146,16 +146,7 @@ struct TcArgs {
   int64_t plane_a;  // bytes between digit planes of the A panels
   const int8_t* pan_b;
   int64_t plane_b;
-  const int32_t* rc_first;
-  const int32_t* rc_atoms;
-  const int32_t* cc_first;
-  const int32_t* cc_atoms;
-  const int8_t* row_bs;  // C (= A) row block sizes
-  const int8_t* col_bs;  // C (= B) column block sizes
-  const int64_t* rbase;  // first element row of every A row atom
-  const int64_t* cbase;  // first element column of every B column atom
-  const int* ea;
-  const int* eb;
+  const int32_t* cc_first;  // atoms before every column cluster
   // C blocks of every tile: tile t owns blist[lbase[t] .. lbase[t + 1]),
   // each (C block index, geometry, data offset low, high word)
   const int4* blist;
@@ -831,21 +822,32 @@ __global__ void k_tc_digits_b(int32_t n_rows, const int64_t* __restrict__ row_p,
   }
 }
 
+// Tiles are numbered, and so processed, by groups of kRowGroup row clusters,
+// inside a group by column cluster, then row cluster: the tiles in flight
+// share A and B panels (1,536 waters: 5.66 -> 5.54 ms; groups of 4 or 16 the same).
+constexpr int kRowGroup = 8;
+__device__ __forceinline__ int64_t tile_slot(int I, int J, int32_t n_cc) {
+  return ((int64_t)(I / kRowGroup) * n_cc + J) * kRowGroup + I % kRowGroup;
+}
+
 // Tile flags: (row cluster, column cluster) pairs holding a C block.
 __global__ void k_tc_tile_flags(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
                                 const int32_t* __restrict__ rcl, const int32_t* __restrict__ ccl, int32_t n_cc,
                                 int64_t* __restrict__ flag) {
   const int lane = threadIdx.x & 31;
   for (int64_t i = global_warp(); i < n_rows; i += grid_warps()) {
-    const int64_t I = rcl[i];
-    for (int64_t b = row_p[i] + lane; b < row_p[i + 1]; b += 32) flag[I * n_cc + ccl[col[b]]] = 1;
+    const int I = rcl[i];
+    for (int64_t b = row_p[i] + lane; b < row_p[i + 1]; b += 32) flag[tile_slot(I, ccl[col[b]], n_cc)] = 1;
   }
 }
 
 __global__ void k_tc_tile_list(int64_t n_map, int32_t n_cc, const int64_t* __restrict__ flag,
                                const int64_t* __restrict__ pos, int2* __restrict__ tiles) {
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n_map; x += (int64_t)gridDim.x * blockDim.x)
-    if (flag[x]) tiles[pos[x]] = make_int2((int)(x / n_cc), (int)(x % n_cc));
+    if (flag[x]) {
+      const int64_t g = x / kRowGroup;
+      tiles[pos[x]] = make_int2((int)(g / n_cc) * kRowGroup + (int)(x % kRowGroup), (int)(g % n_cc));
+    }
 }
 
 // C blocks of every tile.  Count pass: blocks per tile.  Fill pass: one
@@ -863,11 +865,11 @@ __global__ void k_tc_tile_blocks(int32_t n_rows, const int64_t* __restrict__ row
                                  const int64_t* __restrict__ lbase, int4* __restrict__ blist) {
   const int lane = threadIdx.x & 31;
   for (int64_t i = global_warp(); i < n_rows; i += grid_warps()) {
-    const int64_t I = rcl[i];
+    const int I = rcl[i];
     const int geo_r = roff[i] | ((int)row_bs[i] << 7) | (ratom[i] << 14);
     for (int64_t b = row_p[i] + lane; b < row_p[i + 1]; b += 32) {
       const int j = col[b];
-      const int64_t t = pos[I * n_cc + ccl[j]];
+      const int64_t t = pos[tile_slot(I, ccl[j], n_cc)];
       const int64_t slot = (int64_t)atomicAdd(reinterpret_cast<unsigned long long*>(&cnt[t]), 1ull);
       if (FILL) {
         const int geo = geo_r | (catom[j] << 19);
@@ -990,51 +992,225 @@ __global__ void k_tc_tile_stats(int64_t n_tiles, const int64_t* __restrict__ cnt
 }
 
 // Exponent of every tile row / column of every cluster (0 for padding).
-__global__ void k_tc_cluster_exp(int64_t n, const int64_t* __restrict__ elem, const int* __restrict__ e,
+__global__ void k_tc_cluster_exp(int64_t n, const int32_t* __restrict__ elem, const int* __restrict__ e,
                                  int32_t* __restrict__ out) {
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x)
     out[x] = elem[x] >= 0 ? e[elem[x]] : 0;
 }
 
 // ---- host ----------------------------------------------------------------------------------
-struct Clusters {
+// Clusters of nearby atoms.  A tile's inner dimension is the union of what its
+// atoms couple to, so its work grows with the extent of its clusters; cutting
+// the processing order (a Morton curve) into runs leaves clusters that straddle
+// the curve's jumps.  One warp holds the next 256 unplaced atoms of the order
+// in registers, starts a cluster at the first of them and adds the nearest to
+// the cluster's centre (minimum image) that still fits until none does.  One
+// block per range of the order and operand width: a chain of ~0.2 us steps, run
+// once per order.  1,536 waters, cutoff 7: 13.3 -> 10.1 T tensor operations,
+// tiles 6.68 -> 5.66 ms; 200 waters, cutoff 8: 2.50 -> 1.93 T, 0.95 -> 0.77 ms.
+// (A pool of 64 or 512 gives 10.8 or 9.7 T.)
+constexpr int kPoolLane = 8;       // atoms a lane holds: a pool of 256
+constexpr int kPoolRange = 1024;  // atoms of a range at least: each range ends with one cluster to fill
+
+__global__ void __launch_bounds__(32) k_tc_pool(int32_t n, int32_t ranges, const int32_t* __restrict__ order,
+                                                const float* __restrict__ pos, float bx, float by, float bz,
+                                                const int8_t* __restrict__ bs, int32_t* __restrict__ out) {
+  const int lane = threadIdx.x;
+  const bool cols = blockIdx.y != 0;
+  const int cap = cols ? kN : kM, max_atoms = cols ? kMaxColAtoms : kMaxRowAtoms;
+  int next = (int)((int64_t)n * blockIdx.x / ranges);
+  const int end = (int)((int64_t)n * (blockIdx.x + 1) / ranges);
+  int32_t* dst = out + (cols ? n : 0) + next;  // the atoms in cluster order, ~atom where a cluster starts
+  int id[kPoolLane], sz[kPoolLane];
+  unsigned rank[kPoolLane];
+  float x[kPoolLane], y[kPoolLane], z[kPoolLane];
+#pragma unroll
+  for (int j = 0; j < kPoolLane; ++j) {
+    id[j] = -1;
+    rank[j] = 0xffffffffu;
+    sz[j] = 0;
+    x[j] = y[j] = z[j] = 0.f;
+  }
+  for (int placed = 0, total = end - next; placed < total;) {
+    // ---- refill the free slots from the order ----
+#pragma unroll
+    for (int j = 0; j < kPoolLane; ++j) {
+      const unsigned free_ = __ballot_sync(0xffffffffu, id[j] < 0);
+      const int t = next + __popc(free_ & ((1u << lane) - 1u));
+      if (id[j] < 0 && t < end) {
+        const int a = order[t];
+        id[j] = a;
+        rank[j] = (unsigned)t;
+        sz[j] = bs[a];
+      }
+      next = min(end, next + __popc(free_));
+    }
+    // ---- the first unplaced atom starts the cluster; the others' offsets from it ----
+    unsigned first = 0xffffffffu;
+#pragma unroll
+    for (int j = 0; j < kPoolLane; ++j) first = min(first, rank[j]);
+    first = __reduce_min_sync(0xffffffffu, first);
+    const int seed = order[first];
+    const float sx = pos[3 * seed], sy = pos[3 * seed + 1], sz0 = pos[3 * seed + 2];
+    int rows = bs[seed], atoms = 1;
+    if (lane == 0) dst[placed] = ~seed;
+    ++placed;
+#pragma unroll
+    for (int j = 0; j < kPoolLane; ++j) {
+      if (rank[j] == first) {
+        id[j] = -1;
+        rank[j] = 0xffffffffu;
+      }
+      if (id[j] >= 0) {
+        const float dx = pos[3 * id[j]] - sx, dy = pos[3 * id[j] + 1] - sy, dz = pos[3 * id[j] + 2] - sz0;
+        x[j] = dx - bx * rintf(dx / bx);
+        y[j] = dy - by * rintf(dy / by);
+        z[j] = dz - bz * rintf(dz / bz);
+      }
+    }
+    float cx = 0.f, cy = 0.f, cz = 0.f;  // sum of the cluster's offsets
+    while (rows < cap && atoms < max_atoms) {
+      const float inv = 1.f / (float)atoms;
+      const float mx = cx * inv, my = cy * inv, mz = cz * inv;
+      unsigned best = 0xffffffffu;
+#pragma unroll
+      for (int j = 0; j < kPoolLane; ++j) {
+        const float dx = x[j] - mx, dy = y[j] - my, dz = z[j] - mz;
+        const unsigned key = (__float_as_uint(dx * dx + dy * dy + dz * dz) & ~255u) | (unsigned)(lane << 3 | j);
+        if (id[j] >= 0 && rows + sz[j] <= cap) best = min(best, key);
+      }
+      best = __reduce_min_sync(0xffffffffu, best);
+      if (best == 0xffffffffu) break;
+      const int owner = (best >> 3) & 31;
+      int a = 0, b = 0;
+      float ax = 0.f, ay = 0.f, az = 0.f;
+#pragma unroll
+      for (int j = 0; j < kPoolLane; ++j)
+        if ((int)(best & 7u) == j) {
+          a = id[j];
+          b = sz[j];
+          ax = x[j];
+          ay = y[j];
+          az = z[j];
+          if (lane == owner) {
+            id[j] = -1;
+            rank[j] = 0xffffffffu;
+          }
+        }
+      a = __shfl_sync(0xffffffffu, a, owner);
+      rows += __shfl_sync(0xffffffffu, b, owner);
+      cx += __shfl_sync(0xffffffffu, ax, owner);
+      cy += __shfl_sync(0xffffffffu, ay, owner);
+      cz += __shfl_sync(0xffffffffu, az, owner);
+      if (lane == 0) dst[placed] = a;
+      ++placed;
+      ++atoms;
+    }
+  }
+}
+
+// ---- host ----------------------------------------------------------------------------------
+}  // namespace tc
+
+// Clusters of one axis with the tables the kernels read, in one device buffer.
+struct ClusterTab {
+  Ctx* ctx = nullptr;
+  char* buf = nullptr;
   int32_t n = 0;
-  std::vector<int32_t> of, idx, off, first, atoms;
+  bool cols = false;
+  std::vector<int8_t> bs;       // the block sizes it was made for
+  int32_t *of = nullptr, *idx = nullptr, *off = nullptr;  // [atoms] cluster, index and first element in it
+  // rows: [n * kM] (row atom << 16 | element << 8 | block size) of every tile
+  // row, -1 for padding; columns: [n * kMaxColAtoms] first tile column |
+  // width << 8 of every column atom
+  int32_t* desc = nullptr;
+  int32_t* elem = nullptr;      // [n * kM or kN] element row / column of the matrix, -1 for padding
+  int32_t* first = nullptr;     // [n + 1] atoms before the cluster
+  ~ClusterTab() {
+    if (buf) cudaFreeAsync(buf, ctx->stream);
+  }
 };
 
-// Greedy cut of `order` into clusters of at most max_rows rows and max_atoms atoms.
-static Clusters make_clusters(const std::vector<int32_t>& order, const std::vector<int8_t>& bs, int max_rows,
-                              int max_atoms) {
-  Clusters c;
-  const size_t n = bs.size();
-  c.of.assign(n, 0);
-  c.idx.assign(n, 0);
-  c.off.assign(n, 0);
+namespace tc {
+
+// Cuts `order` into clusters of at most max_rows rows and max_atoms atoms, and
+// before every complemented atom of it.
+static int32_t make_clusters(Ctx* ctx, const int32_t* order, const std::vector<int8_t>& bs, bool cols,
+                             std::shared_ptr<ClusterTab>* out) {
+  const int max_rows = cols ? kN : kM, max_atoms = cols ? kMaxColAtoms : kMaxRowAtoms;
+  const int64_t n = (int64_t)bs.size();
+  auto t = std::make_shared<ClusterTab>();
+  t->ctx = ctx;
+  t->cols = cols;
+  t->bs = bs;
+  std::vector<int32_t> h(3 * n), base(n + 1, 0), desc, elem, first;
+  int32_t *of = h.data(), *idx = of + n, *off = idx + n;
+  for (int64_t a = 0; a < n; ++a) base[a + 1] = base[a] + bs[a];
   int rows = 0, atoms = 0;
-  for (size_t t = 0; t < order.size(); ++t) {
-    const int a = order[t], b = bs[a];
-    if (c.first.empty() || rows + b > max_rows || atoms == max_atoms) {
-      c.first.push_back((int32_t)c.atoms.size());
-      rows = 0;
-      atoms = 0;
+  for (int64_t p = 0; p < n; ++p) {
+    const bool head = order[p] < 0;
+    const int a = head ? ~order[p] : order[p], b = bs[a];
+    if (p == 0 || head || rows + b > max_rows || atoms == max_atoms) {
+      ++t->n;
+      first.push_back((int32_t)p);
+      desc.resize((size_t)t->n * (cols ? kMaxColAtoms : kM), cols ? 0 : -1);
+      elem.resize((size_t)t->n * max_rows, -1);
+      rows = atoms = 0;
     }
-    c.of[a] = (int32_t)c.first.size() - 1;
-    c.idx[a] = atoms;
-    c.off[a] = rows;
-    c.atoms.push_back(a);
+    const int64_t I = t->n - 1;
+    of[a] = (int32_t)I;
+    idx[a] = atoms;
+    off[a] = rows;
+    if (cols) desc[I * kMaxColAtoms + atoms] = rows | (b << 8);
+    for (int e = 0; e < b; ++e) {
+      if (!cols) desc[I * kM + rows + e] = (atoms << 16) | (e << 8) | b;
+      elem[I * max_rows + rows + e] = base[a] + e;
+    }
     rows += b;
     ++atoms;
   }
-  c.n = (int32_t)c.first.size();
-  c.first.push_back((int32_t)c.atoms.size());
-  return c;
+  h.insert(h.end(), desc.begin(), desc.end());
+  h.insert(h.end(), elem.begin(), elem.end());
+  first.push_back((int32_t)n);
+  h.insert(h.end(), first.begin(), first.end());
+  LAMB_TRY(dalloc(ctx, &t->buf, (int64_t)(h.size() * sizeof(int32_t))));
+  LAMB_CUDA(ctx, cudaMemcpyAsync(t->buf, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
+  t->of = reinterpret_cast<int32_t*>(t->buf);
+  t->idx = t->of + n;
+  t->off = t->idx + n;
+  t->desc = t->off + n;
+  t->elem = t->desc + desc.size();
+  t->first = t->elem + elem.size();
+  *out = std::move(t);
+  return LAMB_GPU_OK;
 }
 
-template <typename T>
-static int32_t upload_vec(Ctx* ctx, const std::vector<T>& v, T** d) {
-  LAMB_TRY(dalloc(ctx, d, std::max<int64_t>((int64_t)v.size(), 1)));
-  if (!v.empty()) LAMB_CUDA(ctx, cudaMemcpyAsync(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, ctx->stream));
-  return LAMB_GPU_OK;
+// Row clusters of A and, if asked for, column clusters of the same atoms: kept with the matrix.
+static int32_t ensure_clusters(Ctx* ctx, DevMatrix* A, bool cols) {
+  auto have = [&](const std::shared_ptr<ClusterTab>& t) { return t && t->bs == A->h_row_bs; };
+  if (have(A->rclu) && (!cols || have(A->cclu))) return LAMB_GPU_OK;
+  const int32_t n = A->n_rows;
+  std::vector<int32_t> ord(2 * (size_t)n);
+  if ((int64_t)A->h_pos.size() == 3ll * n && A->order) {
+    float* d_pos = nullptr;
+    int32_t* d_out = nullptr;
+    LAMB_TRY(dalloc(ctx, &d_pos, 3ll * n));
+    LAMB_TRY(dalloc(ctx, &d_out, 2ll * n));
+    LAMB_CUDA(ctx, cudaMemcpyAsync(d_pos, A->h_pos.data(), sizeof(float) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
+    const int ranges = std::max(1, n / kPoolRange);
+    k_tc_pool<<<dim3((unsigned)ranges, cols ? 2 : 1), 32, 0, ctx->stream>>>(n, ranges, A->order, d_pos, A->box[0], A->box[1],
+                                                                 A->box[2], A->row_bs, d_out);
+    LAMB_LAUNCHED(ctx);
+    LAMB_CUDA(ctx, cudaMemcpyAsync(ord.data(), d_out, sizeof(int32_t) * (cols ? 2 : 1) * n, cudaMemcpyDeviceToHost, ctx->stream));
+    LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    dfree(ctx, d_pos);
+    dfree(ctx, d_out);
+  } else {
+    std::copy(A->h_order.begin(), A->h_order.end(), ord.begin());
+    std::copy(A->h_order.begin(), A->h_order.end(), ord.begin() + n);
+  }
+  LAMB_TRY(make_clusters(ctx, ord.data(), A->h_row_bs, false, &A->rclu));
+  return !cols ? LAMB_GPU_OK : make_clusters(ctx, ord.data() + n, A->h_row_bs, true, &A->cclu);
 }
 
 // Device buffers of one call, released (stream-ordered) when it returns.
@@ -1048,12 +1224,6 @@ struct Bufs {
   template <typename T>
   int32_t alloc(T** d, int64_t n) {
     LAMB_TRY(dalloc(ctx, d, std::max<int64_t>(n, 1)));
-    p.push_back(*d);
-    return LAMB_GPU_OK;
-  }
-  template <typename T>
-  int32_t up(const std::vector<T>& v, T** d) {
-    LAMB_TRY(upload_vec(ctx, v, d));
     p.push_back(*d);
     return LAMB_GPU_OK;
   }
@@ -1078,51 +1248,24 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   if (C->nnz == 0) { *ran = true; return LAMB_GPU_OK; }
   // ---- clusters (host, from the row processing order) ----
   if ((int)A->h_order.size() != A->n_rows) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_INTERNAL_ERROR, "mixed: row order missing");
-  const Clusters rc = make_clusters(A->h_order, A->h_row_bs, kM, kMaxRowAtoms);
-  std::vector<int32_t> corder(B->n_cols);
-  if (B->n_cols == A->n_rows && B->h_col_bs == A->h_row_bs)
-    corder = A->h_order;
-  else
-    std::iota(corder.begin(), corder.end(), 0);
-  const Clusters cc = make_clusters(corder, B->h_col_bs, kN, kMaxColAtoms);
+  // columns of the rows' atoms share their order and coordinates
+  const bool same = B->n_cols == A->n_rows && B->h_col_bs == A->h_row_bs;
+  LAMB_TRY(ensure_clusters(ctx, A, same));
+  std::shared_ptr<ClusterTab> ccp = A->cclu;
+  if (!same) {
+    std::vector<int32_t> ident(B->n_cols);
+    std::iota(ident.begin(), ident.end(), 0);
+    LAMB_TRY(make_clusters(ctx, ident.data(), B->h_col_bs, true, &ccp));
+  }
+  const ClusterTab &rc = *A->rclu, &cc = *ccp;
   const int32_t nk = A->n_cols, W = (nk + 31) / 32;
   Bufs m{ctx, {}};
-  int32_t *d_rcl, *d_ratom, *d_roff, *d_rcf, *d_rca, *d_ccl, *d_catom, *d_coff, *d_ccf, *d_cca;
-  LAMB_TRY(m.up(rc.of, &d_rcl)); LAMB_TRY(m.up(rc.idx, &d_ratom)); LAMB_TRY(m.up(rc.off, &d_roff));
-  LAMB_TRY(m.up(rc.first, &d_rcf)); LAMB_TRY(m.up(rc.atoms, &d_rca));
-  LAMB_TRY(m.up(cc.of, &d_ccl)); LAMB_TRY(m.up(cc.idx, &d_catom)); LAMB_TRY(m.up(cc.off, &d_coff));
-  LAMB_TRY(m.up(cc.first, &d_ccf)); LAMB_TRY(m.up(cc.atoms, &d_cca));
-  // per-cluster tables of the epilogue: row and column-atom descriptors, row and column exponents
-  std::vector<int32_t> h_rc_row((size_t)rc.n * kM, -1), h_cc_ab((size_t)cc.n * kMaxColAtoms, 0);
-  std::vector<int64_t> h_rc_elem((size_t)rc.n * kM, -1), h_cc_elem((size_t)cc.n * kN, -1);
-  {
-    std::vector<int64_t> rb(A->n_rows + 1, 0), cb(B->n_cols + 1, 0);
-    for (int i = 0; i < A->n_rows; ++i) rb[i + 1] = rb[i] + A->h_row_bs[i];
-    for (int j = 0; j < B->n_cols; ++j) cb[j + 1] = cb[j] + B->h_col_bs[j];
-    for (int I = 0; I < rc.n; ++I)
-      for (int a = 0; a < rc.first[I + 1] - rc.first[I]; ++a) {
-        const int atom = rc.atoms[rc.first[I] + a], b = A->h_row_bs[atom], o = rc.off[atom];
-        for (int pe = 0; pe < b; ++pe) {
-          h_rc_row[(size_t)I * kM + o + pe] = (a << 16) | (pe << 8) | b;
-          h_rc_elem[(size_t)I * kM + o + pe] = rb[atom] + pe;
-        }
-      }
-    for (int J = 0; J < cc.n; ++J)
-      for (int b = 0; b < cc.first[J + 1] - cc.first[J]; ++b) {
-        const int atom = cc.atoms[cc.first[J] + b], w = B->h_col_bs[atom], o = cc.off[atom];
-        h_cc_ab[(size_t)J * kMaxColAtoms + b] = o | (w << 8);
-        for (int q = 0; q < w; ++q) h_cc_elem[(size_t)J * kN + o + q] = cb[atom] + q;
-      }
-  }
-  int32_t *d_rc_row, *d_cc_ab, *d_rc_exp, *d_cc_exp;
-  int64_t *d_rc_elem, *d_cc_elem;
-  LAMB_TRY(m.up(h_rc_row, &d_rc_row));
-  LAMB_TRY(m.up(h_cc_ab, &d_cc_ab));
-  LAMB_TRY(m.up(h_rc_elem, &d_rc_elem)); LAMB_TRY(m.up(h_cc_elem, &d_cc_elem));
+  const int32_t *d_rcl = rc.of, *d_ratom = rc.idx, *d_roff = rc.off, *d_ccl = cc.of, *d_catom = cc.idx, *d_coff = cc.off;
+  int32_t *d_rc_exp, *d_cc_exp;
   LAMB_TRY(m.alloc(&d_rc_exp, (int64_t)rc.n * kM)); LAMB_TRY(m.alloc(&d_cc_exp, (int64_t)cc.n * kN));
-  k_tc_cluster_exp<<<grid_for((int64_t)rc.n * kM), 256, 0, ctx->stream>>>((int64_t)rc.n * kM, d_rc_elem, mp.ea, d_rc_exp);
+  k_tc_cluster_exp<<<grid_for((int64_t)rc.n * kM), 256, 0, ctx->stream>>>((int64_t)rc.n * kM, rc.elem, mp.ea, d_rc_exp);
   LAMB_LAUNCHED(ctx);
-  k_tc_cluster_exp<<<grid_for((int64_t)cc.n * kN), 256, 0, ctx->stream>>>((int64_t)cc.n * kN, d_cc_elem, mp.eb, d_cc_exp);
+  k_tc_cluster_exp<<<grid_for((int64_t)cc.n * kN), 256, 0, ctx->stream>>>((int64_t)cc.n * kN, cc.elem, mp.eb, d_cc_exp);
   LAMB_LAUNCHED(ctx);
   // ---- inner-atom bitmaps and panel row offsets ----
   uint32_t *bma, *bmb;
@@ -1147,7 +1290,7 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   LAMB_TRY(exclusive_scan_i64(ctx, tra, basea, rc.n + 1));
   LAMB_TRY(exclusive_scan_i64(ctx, trb, baseb, cc.n + 1));
   // ---- tiles: cluster pairs holding a C block ----
-  const int64_t n_map = (int64_t)rc.n * cc.n;
+  const int64_t n_map = (int64_t)(rc.n + kRowGroup - 1) / kRowGroup * kRowGroup * cc.n;
   int64_t *flag, *pos;
   LAMB_TRY(m.alloc(&flag, n_map + 1)); LAMB_TRY(m.alloc(&pos, n_map + 1));
   LAMB_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(int64_t) * (size_t)(n_map + 1), ctx->stream));
@@ -1156,10 +1299,10 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   LAMB_LAUNCHED(ctx);
   LAMB_TRY(exclusive_scan_i64(ctx, flag, pos, n_map + 1));
   // panel rows of A and B and the tile count in one read-back
-  int64_t h_sizes[3] = {0, 0, 0};
-  LAMB_CUDA(ctx, cudaMemcpyAsync(&h_sizes[0], basea + rc.n, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(&h_sizes[1], baseb + cc.n, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync(&h_sizes[2], pos + n_map, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  auto* h_sizes = reinterpret_cast<volatile int64_t*>(ctx->pin + kPinTc);
+  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)&h_sizes[0], basea + rc.n, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)&h_sizes[1], baseb + cc.n, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)&h_sizes[2], pos + n_map, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   const int64_t ra = h_sizes[0], rb = h_sizes[1], n_tiles = h_sizes[2];
   if (ra + 1 > kRowMask || rb + 1 > INT_MAX) return LAMB_GPU_OK;  // panel rows beyond the entry format: not run
@@ -1215,8 +1358,8 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   k_tc_tile_stats<<<grid_for(n_tiles, 256), 256, 0, ctx->stream>>>(n_tiles, ecnt, krows, d_stats);
   LAMB_LAUNCHED(ctx);
   LAMB_CUDA(ctx, cudaMemcpyAsync(d_stats + 3, ebase + n_tiles, sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->stream));
-  unsigned long long h_stats[4] = {0, 0, 0, 0};
-  LAMB_CUDA(ctx, cudaMemcpyAsync(h_stats, d_stats, sizeof(h_stats), cudaMemcpyDeviceToHost, ctx->stream));
+  auto* h_stats = reinterpret_cast<volatile unsigned long long*>(ctx->pin + kPinTc + 3);
+  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)h_stats, d_stats, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   const int64_t max_ent = (int64_t)h_stats[0], max_rows = (int64_t)h_stats[1], n_ent = (int64_t)h_stats[3];
   *tensor_ops = (double)h_stats[2] * (kS * (kS + 1) / 2) * 2.0 * kM * kN * kK;
@@ -1234,19 +1377,19 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   TcArgs g{};
   g.tiles = tiles; g.n_tiles = n_tiles; g.ent_base = ebase; g.ent_cnt = ecnt; g.krows = krows; g.ent = ent;
   g.pan_a = pan_a; g.plane_a = plane_a; g.pan_b = pan_b; g.plane_b = plane_b;
-  g.rc_first = d_rcf; g.rc_atoms = d_rca; g.cc_first = d_ccf; g.cc_atoms = d_cca;
-  g.row_bs = C->row_bs; g.col_bs = C->col_bs; g.rbase = mp.rbase; g.cbase = mp.cbase; g.ea = mp.ea; g.eb = mp.eb;
+  g.cc_first = cc.first;
   g.blist = blist; g.lbase = lbase; g.c_data = C->data; g.c_nrm = c_nrm; g.err = d_err;
-  g.rc_exp = d_rc_exp; g.rc_row = d_rc_row; g.cc_exp = d_cc_exp; g.cc_ab = d_cc_ab;
+  g.rc_exp = d_rc_exp; g.rc_row = rc.desc; g.cc_exp = d_cc_exp; g.cc_ab = cc.desc;
   LAMB_CUDA(ctx, cudaFuncSetAttribute(k_tc_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const int grid = (int)std::min<int64_t>(n_tiles, sms);
   k_tc_tiles<<<grid, kTileThreads, kSmemBytes, ctx->stream>>>(g);
   LAMB_LAUNCHED(ctx);
-  int h_err = 0;
-  LAMB_CUDA(ctx, cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  auto* p_err = reinterpret_cast<volatile int*>(ctx->pin + kPinTc + 7);
+  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)p_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  const int h_err = *p_err;
   if (h_err)
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_INTERNAL_ERROR,
                 "mixed: tensor-core tile kernel stopped (code " + std::to_string(h_err) + ")");
