@@ -33,14 +33,17 @@
 // would skip are included (they are bounded by eps each); the C pattern is
 // the filtered one, so only C blocks of the pattern are written.
 //
-// Kernel roles (one CTA of 352 threads per SM, persistent over the tiles):
+// Kernel roles (one CTA of 512 threads per SM, persistent over the tiles):
 //   warps 0-5  producers: gather the tile's K rows, 32 per pipeline stage
 //              (four warps the A chunks, two warps the B chunks);
-//   warp 6     loads each tile's inner-atom list one tile ahead, allocates
-//              the tensor memory (6 levels x 64 columns in 512) and from one
-//              lane issues nine MMAs (M=128, K=32, N=64..256) per stage,
-//              one per A digit plane and run of up to four B digit planes;
-//   warps 7-10 epilogue: tensor memory -> FP64 staging tile in shared
+//   warp 6     allocates the tensor memory (6 levels x 64 columns in 512) and
+//              from one lane issues nine MMAs (M=128, K=32, N=64..256) per
+//              stage, one per A digit plane and run of up to four B digit
+//              planes;
+//   warp 7     expands the tiles' inner lists (runs of panel rows) into the 32
+//              (A row, B row) pairs of every stage, up to kRing stages ahead
+//              of the producers;
+//   warps 8-15 epilogue: tensor memory -> FP64 staging tile in shared
 //              memory (the six levels of a column recombined exactly in two
 //              int64 sums), then column scaling and per-row partial sums of
 //              squares per column atom; every C block of the tile copied out
@@ -48,6 +51,16 @@
 //              and its norm summed from the row partials.  The tile's block
 //              list (built before the kernel) and exponents are loaded one
 //              tile ahead into registers.
+// What bounds it: the MMAs of a stage take ~665 clocks (the tensor pipe and its
+// operand reads from shared memory, ~590), the copies of a stage ~350 of the
+// producers' time.  With three stages the MMAs waited a third of the time for
+// data; the fourth stage's 36 KB come from the inner lists, which no longer lie
+// in shared memory, and from the row sums, which overwrite the staged columns
+// they came from.  Tiles alone: 200 waters, cutoff 8 (65 stages a tile): 0.73 ->
+// 0.68 ms, 2,850 of the probe's 4,340 TOP/s; 1,536 waters, cutoff 7 (11 stages a
+// tile, bound by the epilogue's ~14 k clocks): 5.54 -> 4.75 ms.  Slower there:
+// storing straight from tensor memory (6.2 ms: it stays occupied), whole blocks
+// by a warp (5.9), eight columns loaded ahead of their stores (6.3).
 // Every wait on an mbarrier is bounded (2 s of %globaltimer); on a timeout
 // the kernel records an error code, every role stops, and the host returns
 // an error status.
@@ -66,17 +79,16 @@ namespace tc {
 
 constexpr int kS = 6;                 // digits per operand
 constexpr int kM = 128, kN = 64, kK = 32;
-constexpr int kStages = 3;
+constexpr int kStages = 4;
+constexpr int kRing = 8;              // stages whose rows are listed ahead
 constexpr int kPlaneA = kK * kM;      // bytes of one digit plane of one stage (A)
 constexpr int kPlaneB = kK * kN;
 constexpr int kStageA = kS * kPlaneA;
 constexpr int kStageB = kS * kPlaneB;
 constexpr int kStageBytes = kStageA + kStageB;  // 36,864: a multiple of 1,024
-constexpr int kMaxEnt = 1024;         // inner-list entries of one tile (runs of consecutive atoms)
 constexpr int kMaxRowAtoms = 32;      // atoms of one row cluster
 constexpr int kMaxColAtoms = 16;      // atoms of one column cluster
 constexpr int kMaxBlocks = kMaxRowAtoms * kMaxColAtoms;  // C blocks of one tile
-constexpr int kPartStride = kMaxColAtoms + 1;  // padded: the rows of a warp hit distinct banks
 // An integer x with |x| < 2^51 added to the bit pattern of 2^52 + 2^51 gives
 // the double 2^52 + 2^51 + x exactly; subtracting that constant leaves x.
 constexpr long long kBias = 0x4338000000000000LL;
@@ -86,9 +98,11 @@ constexpr double kBiasD = 6755399441055744.0;
 constexpr int kExactExp = 500;
 constexpr int kProdWarps = 6;                 // warps 0-5: producers
 constexpr int kProducers = 32 * kProdWarps;
-constexpr int kMmaWarp = kProdWarps;          // warp 6: entry loader and MMA issuer
-constexpr int kEpiWarp0 = kMmaWarp + 1;       // warps 7-10: epilogue
-constexpr int kTileThreads = 32 * (kEpiWarp0 + 4);
+constexpr int kMmaWarp = kProdWarps;          // warp 6: MMA issuer
+constexpr int kListWarp = kMmaWarp + 1;       // warp 7: lists the rows of the stages
+constexpr int kEpiWarp0 = kListWarp + 1;      // warps 8-15: epilogue
+constexpr int kEpiThreads = 2 * kM;           // two threads a tile row
+constexpr int kTileThreads = 32 * kEpiWarp0 + kEpiThreads;
 constexpr int kUnits = 32 * (8 + 4);          // 16-byte (row, chunk) copies of a stage and plane
 static_assert(kUnits % kProducers == 0, "units split evenly over the producers");
 constexpr int kTmemCols = 512;
@@ -102,20 +116,17 @@ __device__ constexpr double kLevelW[kS] = {1.0 / 16129.0, 1.0 / (16129.0 * 254.0
                                           1.0 / (16129.0 * 1057227821024.0)};
 
 enum : int { kErrTimeoutFull = 1, kErrTimeoutEmpty = 2, kErrTimeoutTmemFull = 4, kErrTimeoutTmemEmpty = 8,
-             kErrTimeoutEnt = 16, kErrTimeoutDone = 32, kErrEntries = 64 };
+             kErrTimeoutRows = 16, kErrTimeoutDone = 32 };
 
 // ---- shared-memory layout of the tile kernel --------------------------------------------
 struct __align__(16) TileSmem {
-  // the tile's scaled FP64 values: element (m, n) at m * kN + (n ^ (m % 16))
+  // the tile's scaled FP64 values: element (m, n) at m * kN + (n ^ (m % 16));
+  // once a column atom of a row is written out, its first element holds the
+  // sum of squares of the row over the atom's columns
   double stg[kM * kN];
-  // sum of squares of row m over the columns of column atom b, at m * kPartStride + b
-  double part[kM * kPartStride];
-  // entries of two tiles (the loader fills one while the producers use the other)
-  int32_t ent_a[2][kMaxEnt];
-  int32_t ent_b[2][kMaxEnt];
-  uint16_t ent_pre[2][kMaxEnt + 8];  // first K row of every entry (K rows < 2^16)
-  int32_t ent_n[2];
-  int32_t ent_k[2];  // K rows of the tile
+  // (A panel row, B panel row) of the inner rows of the next stages; A row
+  // kPadRow: zeros, kEndRow: no further stage
+  int2 rows[kRing][kK];
   // epilogue tables of the current tile
   long long boff[kMaxBlocks];     // data offset of C block (row atom a, column atom b) at a * 16 + b, or -1
   int32_t blk_id[kMaxBlocks];     // C blocks of the tile in list order: index in C
@@ -126,14 +137,14 @@ struct __align__(16) TileSmem {
   int32_t n_blk;
   int32_t n_col_atoms;
   unsigned long long bar_full[kStages], bar_empty[kStages];
-  unsigned long long bar_tmem_full, bar_tmem_empty, bar_ent_full[2], bar_ent_empty[2], bar_done;
+  unsigned long long bar_tmem_full, bar_tmem_empty, bar_row_full[kRing], bar_row_empty[kRing], bar_done;
   uint32_t tmem_base;
   int abort;
 };
 
 constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + sizeof(TileSmem) + 1024;  // + alignment slack
 static_assert(kSmemBytes <= 232448, "tile kernel exceeds the shared memory of one CTA");
-static_assert(kMaxKRows < 65536, "entry starts are stored as 16-bit K rows");
+constexpr int kPadRow = -1, kEndRow = -2;
 
 struct TcArgs {
   const int2* tiles;
@@ -281,10 +292,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
       bar_init(&sm->bar_empty[s], 1);
     }
     bar_init(&sm->bar_tmem_full, 1);
-    bar_init(&sm->bar_tmem_empty, 128);
-    for (int b = 0; b < 2; ++b) {
-      bar_init(&sm->bar_ent_full[b], 32);
-      bar_init(&sm->bar_ent_empty[b], kProducers);
+    bar_init(&sm->bar_tmem_empty, kEpiThreads);
+    for (int b = 0; b < kRing; ++b) {
+      bar_init(&sm->bar_row_full[b], 32);
+      bar_init(&sm->bar_row_empty[b], kProdWarps);
     }
     bar_init(&sm->bar_done, 1);
     sm->abort = 0;
@@ -310,92 +321,54 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
     // 0..255 are A (row u / 8, chunk u % 8), 256..383 are B (row v / 4,
     // chunk v % 4): consecutive lanes copy consecutive chunks of one panel
     // row, so a warp reads whole 128-byte (A) or 64-byte (B) rows.
-    int64_t gs = 0;      // stages issued by this CTA so far
-    int64_t local = 0;
-    for (int64_t t = blockIdx.x; t < n_tiles && !sm->abort; t += gridDim.x, ++local) {
-      const int buf = (int)(local & 1);
-      if (!bar_wait(&sm->bar_ent_full[buf], (uint32_t)((local >> 1) & 1), sm, g.err, kErrTimeoutEnt)) break;
-      const int n = sm->ent_n[buf];
-      const int K = sm->ent_k[buf];
-      const int nst = K > 0 ? (K + kK - 1) / kK : 1;
-      const uint16_t* pre = sm->ent_pre[buf];
-      // last entry e with pre[e] <= kk (a binary search; only for stages
-      // where more than 31 entries start)
-      auto find = [&](int kk) {
-        int lo = 0, hi = n - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (pre[mid] <= kk) lo = mid; else hi = mid - 1;
-        }
-        return lo;
-      };
-      int e0 = 0;  // the entry holding the stage's first inner row
-      for (int s = 0; s < nst; ++s, ++gs) {
-        const int stg = (int)(gs % kStages);
-        if (!bar_wait(&sm->bar_empty[stg], (uint32_t)(((gs / kStages) & 1) ^ 1), sm, g.err, kErrTimeoutEmpty)) break;
-        const uint32_t sa = smem_u32(stages + (size_t)stg * kStageBytes);
-        const uint32_t sb = sa + kStageA;
-        // lane r of every producer warp finds the panel rows of the stage's
-        // inner row r; the units take them by shuffle.  Lane j reads the
-        // start of entry e0 + j: the entries starting inside the stage set
-        // one bit each (starts are distinct, every entry has rows), and the
-        // entry of row r is e0 plus the starts at or before it.
-        int my_a = 0, my_b = 0;
-        {
-          const int r0 = s * kK, kk = r0 + lane;
-          const int j = e0 + lane;
-          const int P = j <= n ? (int)pre[j] : 0x10000;
-          const uint32_t mask = __reduce_or_sync(0xffffffffu, lane >= 1 && P < r0 + kK ? 1u << (P - r0) : 0u);
-          const bool at_end = __any_sync(0xffffffffu, lane >= 1 && P == r0 + kK);
-          const bool crowded = __shfl_sync(0xffffffffu, P, 31) < r0 + kK;  // starts beyond the 32 read
-          int e;
-          if (!crowded) {
-            e = e0 + __popc(mask & (0xffffffffu >> (31 - lane)));
-            e0 += __popc(mask) + (at_end ? 1 : 0);
-          } else {
-            e = find(kk < K ? kk : K - 1);
-            e0 = find(r0 + kK < K ? r0 + kK : K - 1);
-          }
-          if (kk < K) {
-            my_a = sm->ent_a[buf][e] + (kk - pre[e]);
-            my_b = sm->ent_b[buf][e] + (kk - pre[e]);
-          }
-        }
+    for (int64_t gs = 0;; ++gs) {
+      const int ring = (int)(gs % kRing), stg = (int)(gs % kStages);
+      if (!bar_wait(&sm->bar_row_full[ring], (uint32_t)((gs / kRing) & 1), sm, g.err, kErrTimeoutRows)) break;
+      int2 prow[kUnits / kProducers];
 #pragma unroll
-        for (int i = 0; i < kUnits / kProducers; ++i) {
-          const int u = pt + kProducers * i;
-          const bool is_a = u < 256;  // uniform over the warp
-          const int row = is_a ? (u >> 3) : ((u - 256) >> 2);
-          const int ch = is_a ? (u & 7) : ((u - 256) & 3);
-          const bool valid = s * kK + row < K;
-          const int64_t prow = __shfl_sync(0xffffffffu, is_a ? my_a : my_b, row);
-          const uint32_t bytes = valid ? 16u : 0u;
-          if (is_a) {
-            const int8_t* src = g.pan_a + prow * 128 + 16 * ch;
-#pragma unroll
-            for (int p = 0; p < kS; ++p) cp16(sa + p * kPlaneA + a_swz(row, ch), src + p * g.plane_a, bytes);
-          } else {
-            const int8_t* src = g.pan_b + prow * 64 + 16 * ch;
-#pragma unroll
-            for (int p = 0; p < kS; ++p) cp16(sb + p * kPlaneB + b_swz(row, ch), src + p * g.plane_b, bytes);
-          }
-        }
-        cp_arrive(&sm->bar_full[stg]);
+      for (int i = 0; i < kUnits / kProducers; ++i) {
+        const int u = pt + kProducers * i;
+        prow[i] = sm->rows[ring][u < 256 ? (u >> 3) : ((u - 256) >> 2)];
       }
-      // the entry buffer of this tile may be refilled once every producer is past it
-      bar_arrive(&sm->bar_ent_empty[buf]);
+      if (prow[0].x == kEndRow) break;
+      __syncwarp();
+      if (lane == 0) bar_arrive(&sm->bar_row_empty[ring]);
+      if (!bar_wait(&sm->bar_empty[stg], (uint32_t)(((gs / kStages) & 1) ^ 1), sm, g.err, kErrTimeoutEmpty)) break;
+      const uint32_t sa = smem_u32(stages + (size_t)stg * kStageBytes);
+      const uint32_t sb = sa + kStageA;
+#pragma unroll
+      for (int i = 0; i < kUnits / kProducers; ++i) {
+        const int u = pt + kProducers * i;
+        const bool is_a = u < 256;  // uniform over the warp
+        const int row = is_a ? (u >> 3) : ((u - 256) >> 2);
+        const int ch = is_a ? (u & 7) : ((u - 256) & 3);
+        const bool valid = prow[i].x >= 0;
+        const uint32_t bytes = valid ? 16u : 0u;
+        if (is_a) {
+          const int8_t* src = g.pan_a + (int64_t)(valid ? prow[i].x : 0) * 128 + 16 * ch;
+#pragma unroll
+          for (int p = 0; p < kS; ++p) cp16(sa + p * kPlaneA + a_swz(row, ch), src + p * g.plane_a, bytes);
+        } else {
+          const int8_t* src = g.pan_b + (int64_t)(valid ? prow[i].y : 0) * 64 + 16 * ch;
+#pragma unroll
+          for (int p = 0; p < kS; ++p) cp16(sb + p * kPlaneB + b_swz(row, ch), src + p * g.plane_b, bytes);
+        }
+      }
+      cp_arrive(&sm->bar_full[stg]);
     }
   } else if (warp >= kEpiWarp0) {
     // ================= epilogue =================
     const int ew = warp & 3;        // tensor-memory lane quarter (warp id mod 4)
     const int et = 32 * ew + lane;  // tile row m
+    const int half = (warp - kEpiWarp0) >> 2;  // columns of the tile this thread stages
+    const int e2 = kM * half + et;
     // Tables of the next tile, loaded into registers while the current tile
     // is written out: this thread's row exponent and row descriptor, the
     // column exponents (threads < kN), column atoms (threads < 16) and
-    // count, block count and up to kMaxBlocks / 128 block-list entries per
+    // count, block count and up to kMaxBlocks / 256 block-list entries per
     // thread.  The list bounds and clusters of the tile after next are
     // loaded one tile earlier still, so no load waits on another.
-    constexpr int kBlkRegs = kMaxBlocks / 128;
+    constexpr int kBlkRegs = kMaxBlocks / kEpiThreads;
     int nx_er = 0, nx_ri = -1, nx_ec = 0, nx_cab = 0, nx_nca = 0, nx_nb = 0;
     int4 nx_b[kBlkRegs];
     int64_t lb_lo = 0, lb_hi = 0;  // list bounds of the tile being prefetched
@@ -409,13 +382,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
       const int I = lb_tile.x, J = lb_tile.y;
       nx_er = g.rc_exp[(int64_t)I * kM + et];
       nx_ri = g.rc_row[(int64_t)I * kM + et];
-      if (et < kN) nx_ec = g.cc_exp[(int64_t)J * kN + et];
-      if (et < kMaxColAtoms) nx_cab = g.cc_ab[(int64_t)J * kMaxColAtoms + et];
+      if (e2 < kN) nx_ec = g.cc_exp[(int64_t)J * kN + e2];
+      if (e2 < kMaxColAtoms) nx_cab = g.cc_ab[(int64_t)J * kMaxColAtoms + e2];
       nx_nca = g.cc_first[J + 1] - g.cc_first[J];
       nx_nb = (int)(lb_hi - lb_lo);
 #pragma unroll
       for (int j = 0; j < kBlkRegs; ++j) {
-        const int k = et + 128 * j;
+        const int k = e2 + kEpiThreads * j;
         nx_b[j] = k < nx_nb ? g.blist[lb_lo + k] : make_int4(0, 0, 0, 0);
       }
     };
@@ -423,20 +396,20 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
     // exponent of the tile lies beyond kExactExp (the same for every thread).
     auto publish = [&]() -> bool {
 #pragma unroll
-      for (int j = 0; j < kBlkRegs; ++j) sm->boff[et + 128 * j] = -1;
-      if (et < kN) {
-        sm->col_exp[et] = nx_ec;
-        sm->col_scale[et] = pow2(nx_ec < -kExactExp || nx_ec > kExactExp ? 0 : nx_ec);
+      for (int j = 0; j < kBlkRegs; ++j) sm->boff[e2 + kEpiThreads * j] = -1;
+      if (e2 < kN) {
+        sm->col_exp[e2] = nx_ec;
+        sm->col_scale[e2] = pow2(nx_ec < -kExactExp || nx_ec > kExactExp ? 0 : nx_ec);
       }
-      if (et < kMaxColAtoms) sm->col_atom[et] = nx_cab;
-      if (et == 0) {
+      if (e2 < kMaxColAtoms) sm->col_atom[e2] = nx_cab;
+      if (e2 == 0) {
         sm->n_blk = nx_nb;
         sm->n_col_atoms = nx_nca;
       }
-      named_sync(2, 128);  // every slot reset before the blocks are entered
+      named_sync(2, kEpiThreads);  // every slot reset before the blocks are entered
 #pragma unroll
       for (int j = 0; j < kBlkRegs; ++j) {
-        const int k = et + 128 * j;
+        const int k = e2 + kEpiThreads * j;
         if (k < nx_nb) {
           const int geo = nx_b[j].y;
           sm->blk_id[k] = nx_b[j].x;
@@ -445,8 +418,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
               (long long)(((uint64_t)(uint32_t)nx_b[j].w << 32) | (uint32_t)nx_b[j].z);
         }
       }
-      const bool w = nx_er < -kExactExp || nx_er > kExactExp || (et < kN && (nx_ec < -kExactExp || nx_ec > kExactExp));
-      return named_sync_or(2, 128, w);
+      const bool w = nx_er < -kExactExp || nx_er > kExactExp || (e2 < kN && (nx_ec < -kExactExp || nx_ec > kExactExp));
+      return named_sync_or(2, kEpiThreads, w);
     };
     int64_t local = 0;
     bool wide = false;
@@ -479,7 +452,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
         const double w2 = kLevelW[2] * rs, w5 = kLevelW[5] * rs;
         const uint32_t lane_base = tmem + ((uint32_t)(32 * ew) << 16);
 #pragma unroll 1
-        for (int c0 = 0; c0 < kN; c0 += 16) {
+        for (int c0 = (kN / 2) * half; c0 < (kN / 2) * (half + 1); c0 += 16) {
           int v[kS][16];
 #pragma unroll
           for (int L = 0; L < kS; ++L) tmem_ld16(lane_base + (uint32_t)(64 * L + c0), v[L]);
@@ -499,18 +472,20 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
         prefetch();
         bounds(t + 2 * (int64_t)gridDim.x);
       }
+      named_sync(2, kEpiThreads);  // both halves of every row are staged
       // ---- write-out: each thread writes its tile row into the C blocks of
-      // its row atom, one column atom after the other (a block's column is
+      // its row atom, one column atom after the other (those that start in its
+      // half of the columns; a block's column is
       // bi consecutive doubles, so a warp's store covers its rows' runs),
       // scaling by the column's power of two, and keeps the row's sum of
       // squares per column atom for the block norms ----
       if (ri >= 0) {
         const int a = ri >> 16, pe = (ri >> 8) & 0xff, bi = ri & 0xff;
         const int nca = sm->n_col_atoms;
-        double* part = sm->part + et * kPartStride;
         for (int b = 0; b < nca; ++b) {
           const int cab = sm->col_atom[b];
           const int c0 = cab & 0xff, bj = cab >> 8;
+          if ((c0 >= kN / 2) != (half != 0)) continue;
           const long long bo = sm->boff[a * kMaxColAtoms + b];
           double sq = 0.0;
           if (bo >= 0) {
@@ -532,104 +507,112 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
               }
             }
           }
-          part[b] = sq;
+          if (bj > 0) row[c0 ^ sw] = sq;
         }
       }
-      named_sync(2, 128);
+      named_sync(2, kEpiThreads);
       // ---- block norms: rows of the block in ascending order ----
       const int nb = sm->n_blk;
-      for (int k = et; k < nb; k += 128) {
+      for (int k = e2; k < nb; k += kEpiThreads) {
         const int geo = sm->blk_geom[k];
-        const int r0 = geo & 127, bi = (geo >> 7) & 127, cb = (geo >> 19) & 15;
+        const int r0 = geo & 127, bi = (geo >> 7) & 127, cab = sm->col_atom[(geo >> 19) & 15];
         double sq = 0.0;
-        for (int pe = 0; pe < bi; ++pe) sq += sm->part[(r0 + pe) * kPartStride + cb];
+        if (cab >> 8)
+          for (int r = r0; r < r0 + bi; ++r) sq += sm->stg[r * kN + ((cab & 0xff) ^ (r & 15))];
         g.c_nrm[sm->blk_id[k]] = __dsqrt_rn(sq);
       }
-      named_sync(2, 128);  // the staging tile and the tables are free again
+      named_sync(2, kEpiThreads);  // the staging tile and the tables are free again
       if (has_next) {
         er = nx_er;
         ri = nx_ri;
         wide = publish();
       }
     }
-  } else {
-    // ================= entry loader (all lanes) and MMA issuer (lane 0) =================
-    // Entries of tile `local` go to buffer local % 2.  The next tile's
-    // entries are loaded into registers when a tile starts and written to
-    // shared memory once the tile's tensor memory is free (the loads fly
-    // meanwhile), before its first MMA, so the producers can move on to the
-    // next tile as soon as they have issued this one.
-    int64_t gs = 0, local_mma = 0;
-    bool ok = true;
-    constexpr int kEntRegs = kMaxEnt / 32;
-    uint2 pre_x[kEntRegs];
-    int pre_n = 0, pre_k = 0, cur_k = 0;
-    // entry count, base and K rows of the tile to prefetch next, loaded one
-    // tile earlier so that the entry loads wait on nothing
-    int64_t nb_cnt = 0, nb_base = 0;
+  } else if (warp == kListWarp) {
+    // ================= rows of the stages =================
+    // The tile's list holds runs (first A panel row | rows << 25, first B panel
+    // row).  A lane holds one run of the current 32, of the next 32 and, on its
+    // way, of the 32 after that, with its first inner row P; the run of a
+    // stage's row r is the last one with P <= r, counted in the bit mask of
+    // the runs that start inside the stage (32 rows: at most 32 of them).
+    int64_t gs = 0, nb_cnt = 0, nb_base = 0;
     int nb_k = 0;
+    bool ok = true;
     auto bounds = [&](int64_t t) {
       nb_cnt = t < n_tiles ? g.ent_cnt[t] : 0;
       nb_base = t < n_tiles ? g.ent_base[t] : 0;
       nb_k = t < n_tiles ? g.krows[t] : 0;
     };
-    auto prefetch = [&]() {
-      pre_n = (int)nb_cnt;
-      pre_k = nb_k;
-#pragma unroll
-      for (int j = 0; j < kEntRegs; ++j) {
-        const int e = lane + 32 * j;
-        pre_x[j] = e < pre_n ? g.ent[nb_base + e] : make_uint2(0u, 0u);
-      }
+    auto slot = [&]() -> int2* {  // the next stage's list, once the producers are past its last use
+      const int ring = (int)(gs % kRing);
+      ok = bar_wait(&sm->bar_row_empty[ring], (uint32_t)(((gs / kRing) & 1) ^ 1), sm, g.err, kErrTimeoutRows);
+      return sm->rows[ring];
     };
-    auto publish = [&](int64_t lidx) -> bool {
-      const int buf = (int)(lidx & 1);
-      if (!bar_wait(&sm->bar_ent_empty[buf], (uint32_t)(((lidx >> 1) & 1) ^ 1), sm, g.err, kErrTimeoutEnt))
-        return false;
-      if (pre_n > kMaxEnt) {
-        atomicOr(g.err, kErrEntries);
-        sm->abort = 1;
-        return false;
-      }
+    auto filled = [&]() {
+      bar_arrive(&sm->bar_row_full[(int)(gs % kRing)]);
+      ++gs;
+    };
+    bounds(blockIdx.x);
+    for (int64_t t = blockIdx.x; ok && t < n_tiles && !*(volatile int*)&sm->abort; t += gridDim.x) {
+      const int n = (int)nb_cnt, K = nb_k;
+      const uint2* __restrict__ ent = g.ent + nb_base;
+      const int nst = K > 0 ? (K + kK - 1) / kK : 1;
+      auto load = [&](int e) { return e < n ? ent[e] : make_uint2(0u, 0u); };
+      uint2 x0 = load(lane), x1 = load(32 + lane), x2 = load(64 + lane);
+      bounds(t + (int64_t)gridDim.x);
       int carry = 0;
-#pragma unroll
-      for (int j = 0; j < kEntRegs; ++j) {
-        if (32 * j >= pre_n) break;
-        const int e = lane + 32 * j;
-        const uint2 x = pre_x[j];
-        const int bk = (int)(x.x >> 25);
-        const int incl = warp_incl_scan(bk, lane);
-        if (e < pre_n) {
-          sm->ent_a[buf][e] = (int32_t)(x.x & kRowMask);
-          sm->ent_b[buf][e] = (int32_t)x.y;
-          sm->ent_pre[buf][e] = (uint16_t)(carry + incl - bk);
-        }
+      auto place = [&](const uint2& x) {
+        const int cnt = (int)(x.x >> 25);
+        const int incl = warp_incl_scan(cnt, lane);
+        const int P = cnt ? carry + incl - cnt : INT_MAX / 2;
         carry += __shfl_sync(0xffffffffu, incl, 31);
+        return P;
+      };
+      int p0 = place(x0), p1 = place(x1);
+      int base = 0, started = 0;  // first run held; runs that start before the stage
+      for (int s = 0; s < nst; ++s) {
+        const int r0 = s * kK;
+        const unsigned d0 = (unsigned)(p0 - r0), d1 = (unsigned)(p1 - r0);
+        const unsigned mask =
+            __reduce_or_sync(0xffffffffu, (d0 < (unsigned)kK ? 1u << d0 : 0u) | (d1 < (unsigned)kK ? 1u << d1 : 0u));
+        const int e = started + __popc(mask & ((2u << lane) - 1u)) - 1 - base;
+        const int from = e & 31;
+        const bool first = e < 32;
+        const uint32_t a0 = __shfl_sync(0xffffffffu, x0.x, from), a1 = __shfl_sync(0xffffffffu, x1.x, from);
+        const uint32_t b0 = __shfl_sync(0xffffffffu, x0.y, from), b1 = __shfl_sync(0xffffffffu, x1.y, from);
+        const int q0 = __shfl_sync(0xffffffffu, p0, from), q1 = __shfl_sync(0xffffffffu, p1, from);
+        const int in = r0 + lane - (first ? q0 : q1);
+        int2* list = slot();
+        if (!ok) break;
+        list[lane] = r0 + lane < K ? make_int2((int)((first ? a0 : a1) & kRowMask) + in, (int)(first ? b0 : b1) + in)
+                                   : make_int2(kPadRow, 0);
+        filled();
+        started += __popc(mask);
+        if (started - 1 - base >= 32) {  // the next stage's first row lies in the second 32
+          x0 = x1;
+          p0 = p1;
+          x1 = x2;
+          p1 = place(x1);
+          base += 32;
+          x2 = load(base + 64 + lane);
+        }
       }
-      if (lane == 0) {
-        sm->ent_pre[buf][pre_n] = (uint16_t)carry;
-        sm->ent_n[buf] = pre_n;
-        sm->ent_k[buf] = pre_k;
-      }
-      __syncwarp();
-      bar_arrive(&sm->bar_ent_full[buf]);
-      return true;
-    };
-    if ((int64_t)blockIdx.x < n_tiles) {
-      bounds(blockIdx.x);
-      prefetch();
-      bounds(blockIdx.x + (int64_t)gridDim.x);
-      ok = publish(0);
     }
-    for (int64_t t = blockIdx.x; ok && t < n_tiles && !sm->abort; t += gridDim.x, ++local_mma) {
-      const bool has_next = t + gridDim.x < n_tiles;
-      cur_k = pre_k;  // K rows of tile t (published with its entries)
-      if (has_next) {
-        prefetch();
-        bounds(t + 2 * (int64_t)gridDim.x);
+    if (ok) {
+      int2* list = slot();
+      if (ok) {
+        list[lane] = make_int2(kEndRow, 0);
+        filled();
       }
-      bool published = !has_next;
-      const int K = cur_k;
+    }
+  } else {
+    // ================= MMA issuer (lane 0) =================
+    int64_t gs = 0, local_mma = 0;
+    bool ok = true;
+    int next_k = (int64_t)blockIdx.x < n_tiles ? g.krows[blockIdx.x] : 0;  // K rows, loaded one tile ahead
+    for (int64_t t = blockIdx.x; ok && t < n_tiles && !*(volatile int*)&sm->abort; t += gridDim.x, ++local_mma) {
+      const int K = next_k;
+      next_k = t + gridDim.x < n_tiles ? g.krows[t + gridDim.x] : 0;
       const int nst = K > 0 ? (K + kK - 1) / kK : 1;
       // tensor memory is free once the epilogue has read the previous tile
       if (!bar_wait(&sm->bar_tmem_empty, (uint32_t)((local_mma & 1) ^ 1), sm, g.err, kErrTimeoutTmemEmpty)) break;
@@ -662,10 +645,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
           mma_commit(&sm->bar_empty[stg]);
         }
         __syncwarp();
-        if (!published) {  // after the tile's first MMAs: the next tile's entries (loaded meanwhile)
-          published = true;
-          if (!(ok = publish(local_mma + 1))) break;
-        }
       }
       if (!ok) break;
       if (lane == 0) mma_commit(&sm->bar_tmem_full);
@@ -971,23 +950,19 @@ __global__ void __launch_bounds__(256) k_tc_tile_k(int64_t n_tiles, const int2* 
 
 // Largest inner-atom count and K of any tile, and the pipeline stages of
 // all tiles (ceil(K / 32), at least one), into out[0..2].
-__global__ void k_tc_tile_stats(int64_t n_tiles, const int64_t* __restrict__ cnt, const int32_t* __restrict__ rows,
-                                unsigned long long* __restrict__ out) {
-  long long me = 0, mr = 0, st = 0;
+__global__ void k_tc_tile_stats(int64_t n_tiles, const int32_t* __restrict__ rows, unsigned long long* __restrict__ out) {
+  long long mr = 0, st = 0;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n_tiles; t += (int64_t)gridDim.x * blockDim.x) {
-    me = max(me, (long long)cnt[t]);
     mr = max(mr, (long long)rows[t]);
     st += rows[t] > 0 ? (rows[t] + kK - 1) / kK : 1;
   }
   for (int o = 16; o; o >>= 1) {
-    me = max(me, __shfl_xor_sync(0xffffffffu, me, o));
     mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, o));
     st += __shfl_xor_sync(0xffffffffu, st, o);
   }
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(&out[0], (unsigned long long)me);
-    atomicMax(&out[1], (unsigned long long)mr);
-    atomicAdd(&out[2], (unsigned long long)st);
+    atomicMax(&out[0], (unsigned long long)mr);
+    atomicAdd(&out[1], (unsigned long long)st);
   }
 }
 
@@ -1351,19 +1326,19 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
       n_tiles, tiles, W, bma, bmb, wra, wrb, basea, baseb, A->col_bs, ecnt, krows, nullptr, nullptr);
   LAMB_LAUNCHED(ctx);
   LAMB_TRY(exclusive_scan_i64(ctx, ecnt, ebase, n_tiles + 1));
-  // {largest entry count, largest K, stages, entries} in one read-back
+  // {largest K, stages, entries} in one read-back
   unsigned long long* d_stats;
-  LAMB_TRY(m.alloc(&d_stats, 4));
-  LAMB_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 4 * sizeof(unsigned long long), ctx->stream));
-  k_tc_tile_stats<<<grid_for(n_tiles, 256), 256, 0, ctx->stream>>>(n_tiles, ecnt, krows, d_stats);
+  LAMB_TRY(m.alloc(&d_stats, 3));
+  LAMB_CUDA(ctx, cudaMemsetAsync(d_stats, 0, 3 * sizeof(unsigned long long), ctx->stream));
+  k_tc_tile_stats<<<grid_for(n_tiles, 256), 256, 0, ctx->stream>>>(n_tiles, krows, d_stats);
   LAMB_LAUNCHED(ctx);
-  LAMB_CUDA(ctx, cudaMemcpyAsync(d_stats + 3, ebase + n_tiles, sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->stream));
+  LAMB_CUDA(ctx, cudaMemcpyAsync(d_stats + 2, ebase + n_tiles, sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->stream));
   auto* h_stats = reinterpret_cast<volatile unsigned long long*>(ctx->pin + kPinTc + 3);
-  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)h_stats, d_stats, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
+  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)h_stats, d_stats, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  const int64_t max_ent = (int64_t)h_stats[0], max_rows = (int64_t)h_stats[1], n_ent = (int64_t)h_stats[3];
-  *tensor_ops = (double)h_stats[2] * (kS * (kS + 1) / 2) * 2.0 * kM * kN * kK;
-  if (max_ent > kMaxEnt || max_rows > kMaxKRows) return LAMB_GPU_OK;  // outside the kernel's limits: not run
+  const int64_t max_rows = (int64_t)h_stats[0], n_ent = (int64_t)h_stats[2];
+  *tensor_ops = (double)h_stats[1] * (kS * (kS + 1) / 2) * 2.0 * kM * kN * kK;
+  if (max_rows > kMaxKRows) return LAMB_GPU_OK;  // outside the kernel's limits: not run
   uint2* ent;
   LAMB_TRY(m.alloc(&ent, n_ent));
   k_tc_tile_k<true><<<grid_for(32ll * n_tiles, 256), 256, 0, ctx->stream>>>(

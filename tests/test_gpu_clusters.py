@@ -77,3 +77,18 @@ def test_rectangular_clusters(gpu_ctx, m):
     r, k, c = np.array([100, 13, 5]), np.array([13, 5, 5]), np.array([7, 0, 30])
     a, b = _band(rng, 120, 150, r, k), _band(rng, 150, m, k, c)
     _check(gpu_ctx, a, b, _positions(rng, 120, "random"))
+
+
+@pytest.mark.parametrize("sizes", [[1], [3, 1, 2], [33, 31]])
+@pytest.mark.parametrize("runs", [1, 31, 32, 33, 63, 64, 65, 97, 1100])
+def test_inner_runs(gpu_ctx, runs, sizes):
+    """Tiles whose inner list has `runs` runs of panel rows: A couples to every
+    other inner atom, B to all of them, so that no two runs follow on."""
+    rng = np.random.default_rng(runs)
+    n = 2 * runs
+    rows, inner, cols = np.array([13, 5, 5]), np.resize(sizes, n), np.array([7, 9])
+    pa = np.zeros((3, n), bool)
+    pa[:, ::2] = True
+    a = _matrix(rng, rows, inner, pa)
+    b = _matrix(rng, inner, cols, np.ones((n, 2), bool))
+    _check(gpu_ctx, a, b, None)
