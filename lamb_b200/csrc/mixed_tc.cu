@@ -685,53 +685,92 @@ __global__ void k_tc_bitmap(int32_t n_rows, const int64_t* __restrict__ row_p, c
     }
 }
 
-// Per cluster and bitmap word: inner atoms and panel rows (sum of their block
-// sizes) before the word; per cluster the totals.  One warp per cluster.
+// Panel rows and pairs (cluster, inner atom) of every cluster before each bitmap word, and their totals.
 __global__ void k_tc_word_prefix(int32_t n_cl, int32_t W, const uint32_t* __restrict__ bm,
-                                 const int8_t* __restrict__ kbs, int32_t* __restrict__ wrow,
-                                 int64_t* __restrict__ tot_row) {
+                                 const int8_t* __restrict__ kbs, int2* __restrict__ before,
+                                 int64_t* __restrict__ tot_row, int64_t* __restrict__ tot_pair) {
   const int lane = threadIdx.x & 31;
   for (int64_t c = global_warp(); c < n_cl; c += grid_warps()) {
-    int carry = 0;
+    int carry = 0, pairs = 0;
     for (int w0 = 0; w0 < W; w0 += 32) {
       const int w = w0 + lane;
       uint32_t bits = w < W ? bm[c * W + w] : 0u;
+      const int n = __popc(bits);
       int rows = 0;
       while (bits) {
         const int bit = __ffs(bits) - 1;
         bits &= bits - 1u;
         rows += kbs[32 * w + bit];
       }
-      const int incl = warp_incl_scan(rows, lane);
-      if (w < W) wrow[c * W + w] = carry + incl - rows;
+      const int incl = warp_incl_scan(rows, lane), incl_n = warp_incl_scan(n, lane);
+      if (w < W) before[c * W + w] = make_int2(carry + incl - rows, pairs + incl_n - n);
       carry += __shfl_sync(0xffffffffu, incl, 31);
+      pairs += __shfl_sync(0xffffffffu, incl_n, 31);
     }
-    if (lane == 0) tot_row[c] = carry;
+    if (lane == 0) {
+      tot_row[c] = carry;
+      tot_pair[c] = pairs;
+    }
   }
 }
 
-// Panel row of inner atom k within cluster c's panel (relative to its
-// base), by the whole warp: lane b adds the rows of atom 32 (k / 32) + b
-// when its bit is set and below k's.
-__device__ __forceinline__ int64_t panel_row_warp(const uint32_t* __restrict__ bm, const int32_t* __restrict__ wrow,
-                                                  const int8_t* __restrict__ kbs, int64_t c, int32_t W, int k,
-                                                  int lane) {
-  const int w = k >> 5;
-  const uint32_t word = bm[c * W + w];
-  const int add = lane < (k & 31) && ((word >> lane) & 1u) ? kbs[32 * w + lane] : 0;
-  return wrow[c * W + w] + __reduce_add_sync(0xffffffffu, add);
+// Exclusive sums of four short arrays, a CTA each: array i has n[i] values, one after the other.
+struct Sums {
+  int64_t n[4];
+};
+__global__ void __launch_bounds__(1024) k_tc_sums(Sums a, const int64_t* __restrict__ in, int64_t* __restrict__ out) {
+  typedef cub::BlockScan<long long, 1024> BS;
+  __shared__ typename BS::TempStorage ts;
+  const int64_t n = a.n[blockIdx.x];
+  for (int i = 0; i < (int)blockIdx.x; ++i) {
+    in += a.n[i];
+    out += a.n[i];
+  }
+  long long carry = 0;
+  for (int64_t x0 = 0; x0 < n; x0 += 1024) {
+    const int64_t x = x0 + threadIdx.x;
+    long long v = x < n ? in[x] : 0, sum = 0;
+    BS(ts).ExclusiveSum(v, v, sum);
+    __syncthreads();
+    if (x < n) out[x] = carry + v;
+    carry += sum;
+  }
 }
 
-// Writes the S digits of x (|x| < 1) to S planes: |127 x| < 127 and every
-// later t lies in [-127, 127], so each digit fits int8.
-__device__ __forceinline__ void put_digits(int8_t* __restrict__ pan, int64_t plane, int64_t pos, double x) {
-  double t = x * kFirst;
-#pragma unroll
-  for (int p = 0; p < kS; ++p) {
-    const double dg = rint(t);
-    pan[p * plane + pos] = (int8_t)dg;
-    t = (t - dg) * kBase;
+// The pairs: (cluster, inner atom, first panel row, rows).
+__global__ void k_tc_pairs(int32_t n_cl, int32_t W, const uint32_t* __restrict__ bm, const int8_t* __restrict__ kbs,
+                           const int2* __restrict__ before, const int64_t* __restrict__ row_base,
+                           const int64_t* __restrict__ pair_base, int4* __restrict__ pair) {
+  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < (int64_t)n_cl * W;
+       x += (int64_t)gridDim.x * blockDim.x) {
+    const int c = (int)(x / W), w = (int)(x % W);
+    int row = (int)row_base[c] + before[x].x;
+    int4* out = pair + pair_base[c] + before[x].y;
+    for (uint32_t bits = bm[x]; bits; bits &= bits - 1u) {
+      const int k = 32 * w + __ffs(bits) - 1, bk = kbs[k];
+      *out++ = make_int4(c, k, row, bk);
+      row += bk;
+    }
   }
+}
+
+// Where the blocks of every pair lie: data offset of the block of the
+// cluster's atom x at pair * per + x (-1, set before, where it is absent).
+template <bool A_SIDE>
+__global__ void k_tc_pair_blocks(int32_t n_rows, int32_t W, const int64_t* __restrict__ row_p,
+                                 const int32_t* __restrict__ col, const int64_t* __restrict__ off,
+                                 const int32_t* __restrict__ clus, const int32_t* __restrict__ idx,
+                                 const uint32_t* __restrict__ bm, const int2* __restrict__ before,
+                                 const int64_t* __restrict__ pair_base, long long* __restrict__ tab) {
+  constexpr int per = A_SIDE ? kMaxRowAtoms : kMaxColAtoms;
+  const int lane = threadIdx.x & 31;
+  for (int64_t i = global_warp(); i < n_rows; i += grid_warps())
+    for (int64_t b = row_p[i] + lane; b < row_p[i + 1]; b += 32) {
+      const int j = col[b], a = A_SIDE ? (int)i : j, k = A_SIDE ? j : (int)i, c = clus[a];
+      const int64_t x = (int64_t)c * W + (k >> 5);
+      const int64_t pair = pair_base[c] + before[x].y + __popc(bm[x] & ((1u << (k & 31)) - 1u));
+      tab[pair * per + idx[a]] = off[b];
+    }
 }
 
 // x * 2^-e: an exact power-of-two multiply where 2^-e is a normal double
@@ -740,62 +779,110 @@ __device__ __forceinline__ double scale_down(double x, int e) {
   return e > -1000 && e < 1000 ? x * __longlong_as_double((long long)(1023 - e) << 52) : ldexp(x, -e);
 }
 
-// Warps per block row in the digit kernels (memory parallelism across the
-// row's blocks).
-constexpr int kDigitWays = 8;
+// Digit panels: panel row base[c] + row(c, k) + r holds one byte per element row
+// (A, 128) or column (B, 64) of cluster c and digit plane, zero where the block
+// is absent.  A warp writes whole panel rows, pair by pair: its lanes hold the
+// elements lane + 32 j (A; two rows of lane % 16 + 16 j, B), so that loads run
+// along a block's storage, and exchange their four digits with three neighbours
+// for words of four consecutive bytes: one full line stored per plane and row,
+// and no plane to clear beforehand.  The pairs' blocks are listed first (the
+// search for them cost more than the digits).
+// Digits.  s = t + 1.5 2^52 rounds t (|t| <= 127) to the integer digit d in its
+// low bits; 254 (t - d) is one fused operation from t and another, exact, for
+// 254 d: 17 FP64 operations an element.  Bound by instruction issue (about 250 a
+// panel row) and the latency of a pair's first loads.  1,536 waters, all of the
+// preparation, with panels cleared and written byte by byte, block by block:
+// 2.12 -> 1.34 ms (0.39 the A panels, 0.31 B); 200 waters 0.52 -> 0.41 ms.
+constexpr double kRound = 6755399441055744.0;  // 1.5 2^52
 
-// A panels: element (pe, kc) of block (i, k) goes to panel row
-// base[I] + row(I, k) + kc, byte roff[i] + pe of that 128-byte row.  Lanes
-// walk the block in storage order (pe fastest), so they write consecutive
-// bytes of a panel row.
-__global__ void k_tc_digits_a(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
-                              const int64_t* __restrict__ off, const int8_t* __restrict__ row_bs,
-                              const int8_t* __restrict__ kbs, const double* __restrict__ data,
-                              const int32_t* __restrict__ rcl, const int32_t* __restrict__ roff, int32_t W,
-                              const uint32_t* __restrict__ bm, const int32_t* __restrict__ wrow,
-                              const int64_t* __restrict__ base, const int64_t* __restrict__ rbase,
-                              const int* __restrict__ ea, int64_t plane, int8_t* __restrict__ pan) {
-  const int lane = threadIdx.x & 31;
-  // kDigitWays warps per block row, each every kDigitWays-th block of it
-  for (int64_t gw = global_warp(); gw < (int64_t)n_rows * kDigitWays; gw += grid_warps()) {
-    const int64_t i = gw / kDigitWays;
-    const int I = rcl[i], m0 = roff[i], bi = row_bs[i];
-    const int64_t e0 = rbase[i];
-    for (int64_t b = row_p[i] + gw % kDigitWays; b < row_p[i + 1]; b += kDigitWays) {
-      const int k = col[b], bk = kbs[k];
-      const int64_t prow = base[I] + panel_row_warp(bm, wrow, kbs, I, W, k, lane);
-      const double* x = data + off[b];
-      Walk w(bi, lane);
-      for (int e = lane; e < bi * bk; e += 32, w.next())
-        put_digits(pan, plane, (prow + w.major) * 128 + m0 + w.minor, scale_down(x[e], ea[e0 + w.minor]));
-    }
-  }
+// The 4 x 4 bytes of four neighbouring lanes transposed: lane i of them gets byte i of each.
+__device__ __forceinline__ uint32_t transpose4(uint32_t w, int lane) {
+  const uint32_t u = __shfl_xor_sync(0xffffffffu, w, 2);
+  const uint32_t a = (lane & 2) ? __byte_perm(u, w, 0x7632) : __byte_perm(w, u, 0x5410);
+  const uint32_t v = __shfl_xor_sync(0xffffffffu, a, 1);
+  return (lane & 1) ? __byte_perm(v, a, 0x7351) : __byte_perm(a, v, 0x6240);
 }
 
-// B panels: element (kr, q) of block (k, j) goes to panel row
-// base[J] + row(J, k) + kr, byte coff[j] + q of that 64-byte row.  Lanes
-// walk the block row by row (q fastest), so they write consecutive bytes of
-// a panel row (the strided reads stay within the block).
-__global__ void k_tc_digits_b(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
-                              const int64_t* __restrict__ off, const int8_t* __restrict__ kbs,
-                              const int8_t* __restrict__ col_bs, const double* __restrict__ data,
-                              const int32_t* __restrict__ ccl, const int32_t* __restrict__ coff, int32_t W,
-                              const uint32_t* __restrict__ bm, const int32_t* __restrict__ wrow,
-                              const int64_t* __restrict__ base, const int64_t* __restrict__ cbase,
-                              const int* __restrict__ eb, int64_t plane, int8_t* __restrict__ pan) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t gw = global_warp(); gw < (int64_t)n_rows * kDigitWays; gw += grid_warps()) {
-    const int64_t k = gw / kDigitWays;
-    const int bk = kbs[k];
-    for (int64_t b = row_p[k] + gw % kDigitWays; b < row_p[k + 1]; b += kDigitWays) {
-      const int j = col[b], J = ccl[j], n0 = coff[j], bj = col_bs[j];
-      const int64_t prow = base[J] + panel_row_warp(bm, wrow, kbs, J, W, (int)k, lane);
-      const double* x = data + off[b];
-      const int64_t e0 = cbase[j];
-      Walk w(bj, lane);
-      for (int e = lane; e < bk * bj; e += 32, w.next()) {
-        const int q = w.minor, kr = w.major;
-        put_digits(pan, plane, (prow + kr) * 64 + n0 + q, scale_down(x[kr + q * bk], eb[e0 + q]));
+constexpr int kDigitPairs = 4;  // a warp takes: mostly of one cluster
+
+template <bool A_SIDE>
+__global__ void __launch_bounds__(128, 5) k_tc_digits(
+    int64_t n_pairs, const int4* __restrict__ pairs, const long long* __restrict__ tab,
+    const int32_t* __restrict__ geo, const int32_t* __restrict__ exps, const double* __restrict__ data, int64_t plane,
+    int8_t* __restrict__ pan) {
+  constexpr int width = A_SIDE ? kM : kN, lanes = width / 4, per = A_SIDE ? kMaxRowAtoms : kMaxColAtoms;
+  constexpr int rows_at_once = 32 / lanes;
+  const int lane = threadIdx.x & 31, l = lane % lanes, sub = lane / lanes;
+  int have = -1;       // cluster of the scales
+  double scale[4] = {};  // 127 2^-exponent: x times it rounds once, as x 2^-exponent (exact) times 127 does
+  bool wide = false;
+  for (int64_t p0 = global_warp() * kDigitPairs; p0 < n_pairs; p0 += grid_warps() * kDigitPairs) {
+    int4 nxt = pairs[p0];
+    long long nxt_o = tab[p0 * per + lane % per];
+    for (int64_t q = p0; q < min(n_pairs, p0 + kDigitPairs); ++q) {
+      const int c = nxt.x, bk = nxt.w;
+      const int64_t prow = nxt.z;
+      const long long o = nxt_o;
+      if (q + 1 < min(n_pairs, p0 + kDigitPairs)) {
+        nxt = pairs[q + 1];
+        nxt_o = tab[(q + 1) * per + lane % per];
+      }
+      const int32_t* __restrict__ g = geo + (int64_t)c * width + l;
+      const int32_t* __restrict__ ex = exps + (int64_t)c * width + l;
+      if (c != have) {
+        have = c;
+        wide = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int e = ex[lanes * j];
+          wide |= !(e > -1000 && e < 1000);
+          scale[j] = kFirst * __longlong_as_double((long long)(1023 - e) << 52);
+        }
+        wide = __any_sync(0xffffffffu, wide);
+      }
+      const double* src[4];
+      bool some[2] = {false, false};  // any block of the warp's elements 2 h and 2 h + 1
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int gj = g[lanes * j];
+        const long long oj = __shfl_sync(0xffffffffu, o, gj >= 0 ? gj >> 16 : 0);
+        const int e = (gj >> 8) & 0xff;
+        src[j] = gj >= 0 && oj >= 0 ? data + oj + (A_SIDE ? e : e * bk + sub) : nullptr;
+        some[j / 2] |= src[j] != nullptr;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) some[h] = __any_sync(0xffffffffu, some[h]);
+      for (int r0 = 0; r0 < bk; r0 += rows_at_once) {
+        const int r = r0 + sub;
+        double t[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          t[j] = src[j] && r < bk ? *src[j] : 0.0;
+          if (src[j]) src[j] += A_SIDE ? g[lanes * j] & 0xff : rows_at_once;
+        }
+        uint32_t d[kS] = {};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (!some[h]) continue;
+#pragma unroll
+          for (int j = 2 * h; j < 2 * h + 2; ++j)
+            t[j] = !wide ? t[j] * scale[j] : scale_down(t[j], ex[lanes * j]) * kFirst;
+#pragma unroll
+          for (int p = 0; p < kS; ++p)
+#pragma unroll
+            for (int j = 2 * h; j < 2 * h + 2; ++j) {
+              const double s = t[j] + kRound;
+              const int sel = j == 0 ? 0x3214 : j == 1 ? 0x3240 : j == 2 ? 0x3410 : 0x4210;  // byte j
+              d[p] = __byte_perm(d[p], (uint32_t)__double2loint(s), sel);
+              if (p + 1 < kS) t[j] = __fma_rn(t[j], kBase, __fma_rn(s, -kBase, kRound * kBase));
+            }
+        }
+        int8_t* dst = pan + (prow + r) * width + lanes * (lane & 3) + (l & ~3);
+#pragma unroll
+        for (int p = 0; p < kS; ++p) {
+          const uint32_t v = transpose4(d[p], lane);
+          if (r < bk) *reinterpret_cast<uint32_t*>(dst + p * plane) = v;
+        }
       }
     }
   }
@@ -910,7 +997,7 @@ __device__ __forceinline__ int tile_word_entries(uint32_t xa, uint32_t xb, int w
 template <bool FILL>
 __global__ void __launch_bounds__(256) k_tc_tile_k(int64_t n_tiles, const int2* __restrict__ tiles, int32_t W,
                                                    const uint32_t* __restrict__ bma, const uint32_t* __restrict__ bmb,
-                                                   const int32_t* __restrict__ wra, const int32_t* __restrict__ wrb,
+                                                   const int2* __restrict__ wra, const int2* __restrict__ wrb,
                                                    const int64_t* __restrict__ basea, const int64_t* __restrict__ baseb,
                                                    const int8_t* __restrict__ kbs, int64_t* __restrict__ cnt,
                                                    int32_t* __restrict__ rows, const int64_t* __restrict__ ebase,
@@ -932,7 +1019,7 @@ __global__ void __launch_bounds__(256) k_tc_tile_k(int64_t n_tiles, const int2* 
       const uint32_t xa = w < W ? bma[I * W + w] : 0u, xb = w < W ? bmb[J * W + w] : 0u;
       int c = 0;
       if (xa & xb) {
-        const int64_t ar = basea[I] + wra[I * W + w], br = baseb[J] + wrb[J * W + w];
+        const int64_t ar = basea[I] + wra[I * W + w].x, br = baseb[J] + wrb[J * W + w].x;
         c = tile_word_entries<FILL>(xa, xb, w, kbs, ar, br, out, &nrows, &slot[wl]);
       }
       if (!FILL) carry += warp_sum_ll(c);
@@ -1095,10 +1182,8 @@ struct ClusterTab {
   bool cols = false;
   std::vector<int8_t> bs;       // the block sizes it was made for
   int32_t *of = nullptr, *idx = nullptr, *off = nullptr;  // [atoms] cluster, index and first element in it
-  // rows: [n * kM] (row atom << 16 | element << 8 | block size) of every tile
-  // row, -1 for padding; columns: [n * kMaxColAtoms] first tile column |
-  // width << 8 of every column atom
-  int32_t* desc = nullptr;
+  int32_t* geo = nullptr;       // [n * kM or kN] atom << 16 | element << 8 | block size of every tile row / column, -1 for padding
+  int32_t* cab = nullptr;       // columns: [n * kMaxColAtoms] first tile column | width << 8 of every column atom
   int32_t* elem = nullptr;      // [n * kM or kN] element row / column of the matrix, -1 for padding
   int32_t* first = nullptr;     // [n + 1] atoms before the cluster
   ~ClusterTab() {
@@ -1118,7 +1203,7 @@ static int32_t make_clusters(Ctx* ctx, const int32_t* order, const std::vector<i
   t->ctx = ctx;
   t->cols = cols;
   t->bs = bs;
-  std::vector<int32_t> h(3 * n), base(n + 1, 0), desc, elem, first;
+  std::vector<int32_t> h(3 * n), base(n + 1, 0), geo, cab, elem, first;
   int32_t *of = h.data(), *idx = of + n, *off = idx + n;
   for (int64_t a = 0; a < n; ++a) base[a + 1] = base[a] + bs[a];
   int rows = 0, atoms = 0;
@@ -1128,7 +1213,8 @@ static int32_t make_clusters(Ctx* ctx, const int32_t* order, const std::vector<i
     if (p == 0 || head || rows + b > max_rows || atoms == max_atoms) {
       ++t->n;
       first.push_back((int32_t)p);
-      desc.resize((size_t)t->n * (cols ? kMaxColAtoms : kM), cols ? 0 : -1);
+      geo.resize((size_t)t->n * max_rows, -1);
+      if (cols) cab.resize((size_t)t->n * kMaxColAtoms, 0);
       elem.resize((size_t)t->n * max_rows, -1);
       rows = atoms = 0;
     }
@@ -1136,25 +1222,24 @@ static int32_t make_clusters(Ctx* ctx, const int32_t* order, const std::vector<i
     of[a] = (int32_t)I;
     idx[a] = atoms;
     off[a] = rows;
-    if (cols) desc[I * kMaxColAtoms + atoms] = rows | (b << 8);
+    if (cols) cab[I * kMaxColAtoms + atoms] = rows | (b << 8);
     for (int e = 0; e < b; ++e) {
-      if (!cols) desc[I * kM + rows + e] = (atoms << 16) | (e << 8) | b;
+      geo[I * max_rows + rows + e] = (atoms << 16) | (e << 8) | b;
       elem[I * max_rows + rows + e] = base[a] + e;
     }
     rows += b;
     ++atoms;
   }
-  h.insert(h.end(), desc.begin(), desc.end());
-  h.insert(h.end(), elem.begin(), elem.end());
   first.push_back((int32_t)n);
-  h.insert(h.end(), first.begin(), first.end());
+  for (const auto* v : {&geo, &cab, &elem, &first}) h.insert(h.end(), v->begin(), v->end());
   LAMB_TRY(dalloc(ctx, &t->buf, (int64_t)(h.size() * sizeof(int32_t))));
   LAMB_CUDA(ctx, cudaMemcpyAsync(t->buf, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
   t->of = reinterpret_cast<int32_t*>(t->buf);
   t->idx = t->of + n;
   t->off = t->idx + n;
-  t->desc = t->off + n;
-  t->elem = t->desc + desc.size();
+  t->geo = t->off + n;
+  t->cab = t->geo + geo.size();
+  t->elem = t->cab + cab.size();
   t->first = t->elem + elem.size();
   *out = std::move(t);
   return LAMB_GPU_OK;
@@ -1243,27 +1328,29 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   k_tc_cluster_exp<<<grid_for((int64_t)cc.n * kN), 256, 0, ctx->stream>>>((int64_t)cc.n * kN, cc.elem, mp.eb, d_cc_exp);
   LAMB_LAUNCHED(ctx);
   // ---- inner-atom bitmaps and panel row offsets ----
-  uint32_t *bma, *bmb;
-  int32_t *wra, *wrb;
-  int64_t *tra, *trb, *basea, *baseb;
-  LAMB_TRY(m.alloc(&bma, (int64_t)rc.n * W)); LAMB_TRY(m.alloc(&bmb, (int64_t)cc.n * W));
+  int2 *wra, *wrb;
   LAMB_TRY(m.alloc(&wra, (int64_t)rc.n * W)); LAMB_TRY(m.alloc(&wrb, (int64_t)cc.n * W));
-  LAMB_TRY(m.alloc(&tra, rc.n + 1)); LAMB_TRY(m.alloc(&trb, cc.n + 1));
-  LAMB_TRY(m.alloc(&basea, rc.n + 1)); LAMB_TRY(m.alloc(&baseb, cc.n + 1));
-  LAMB_CUDA(ctx, cudaMemsetAsync(bma, 0, sizeof(uint32_t) * (size_t)rc.n * W, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemsetAsync(bmb, 0, sizeof(uint32_t) * (size_t)cc.n * W, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemsetAsync(tra + rc.n, 0, sizeof(int64_t), ctx->stream));
-  LAMB_CUDA(ctx, cudaMemsetAsync(trb + cc.n, 0, sizeof(int64_t), ctx->stream));
+  // panel rows and pairs of every cluster of A, then of B, each with a zero
+  // behind, and the bitmaps; what lies before each cluster
+  const int64_t n_a = rc.n + 1, n_b = cc.n + 1;
+  int64_t *tra, *basea;
+  const int64_t zeroed = sizeof(int64_t) * 2 * (n_a + n_b) + sizeof(uint32_t) * ((int64_t)rc.n + cc.n) * W;
+  LAMB_TRY(m.alloc(&tra, zeroed / 8 + 1));
+  LAMB_TRY(m.alloc(&basea, 2 * (n_a + n_b)));
+  int64_t *tpa = tra + n_a, *trb = tpa + n_a, *tpb = trb + n_b;
+  int64_t *pba = basea + n_a, *baseb = pba + n_a, *pbb = baseb + n_b;
+  uint32_t *bma = reinterpret_cast<uint32_t*>(tpb + n_b), *bmb = bma + (int64_t)rc.n * W;
+  LAMB_CUDA(ctx, cudaMemsetAsync(tra, 0, (size_t)zeroed, ctx->stream));
   k_tc_bitmap<<<grid_for(32ll * A->n_rows, 256), 256, 0, ctx->stream>>>(A->n_rows, A->row_p, A->col, d_rcl, 1, W, bma);
   LAMB_LAUNCHED(ctx);
   k_tc_bitmap<<<grid_for(32ll * B->n_rows, 256), 256, 0, ctx->stream>>>(B->n_rows, B->row_p, B->col, d_ccl, 0, W, bmb);
   LAMB_LAUNCHED(ctx);
-  k_tc_word_prefix<<<grid_for(32ll * rc.n, 256), 256, 0, ctx->stream>>>(rc.n, W, bma, A->col_bs, wra, tra);
+  k_tc_word_prefix<<<grid_for(32ll * rc.n, 256), 256, 0, ctx->stream>>>(rc.n, W, bma, A->col_bs, wra, tra, tpa);
   LAMB_LAUNCHED(ctx);
-  k_tc_word_prefix<<<grid_for(32ll * cc.n, 256), 256, 0, ctx->stream>>>(cc.n, W, bmb, B->row_bs, wrb, trb);
+  k_tc_word_prefix<<<grid_for(32ll * cc.n, 256), 256, 0, ctx->stream>>>(cc.n, W, bmb, B->row_bs, wrb, trb, tpb);
   LAMB_LAUNCHED(ctx);
-  LAMB_TRY(exclusive_scan_i64(ctx, tra, basea, rc.n + 1));
-  LAMB_TRY(exclusive_scan_i64(ctx, trb, baseb, cc.n + 1));
+  k_tc_sums<<<4, 1024, 0, ctx->stream>>>(Sums{{n_a, n_a, n_b, n_b}}, tra, basea);
+  LAMB_LAUNCHED(ctx);
   // ---- tiles: cluster pairs holding a C block ----
   const int64_t n_map = (int64_t)(rc.n + kRowGroup - 1) / kRowGroup * kRowGroup * cc.n;
   int64_t *flag, *pos;
@@ -1273,28 +1360,42 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
                                                                          cc.n, flag);
   LAMB_LAUNCHED(ctx);
   LAMB_TRY(exclusive_scan_i64(ctx, flag, pos, n_map + 1));
-  // panel rows of A and B and the tile count in one read-back
+  // panel rows and pairs of A and B and the tile count
   auto* h_sizes = reinterpret_cast<volatile int64_t*>(ctx->pin + kPinTc);
-  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)&h_sizes[0], basea + rc.n, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)&h_sizes[1], baseb + cc.n, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  LAMB_CUDA(ctx, cudaMemcpyAsync((void*)&h_sizes[2], pos + n_map, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  const int64_t* d_sizes[5] = {basea + rc.n, baseb + cc.n, pba + rc.n, pbb + cc.n, pos + n_map};
+  for (int i = 0; i < 5; ++i)
+    LAMB_CUDA(ctx, cudaMemcpyAsync((void*)&h_sizes[i], d_sizes[i], sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  const int64_t ra = h_sizes[0], rb = h_sizes[1], n_tiles = h_sizes[2];
+  const int64_t ra = h_sizes[0], rb = h_sizes[1], na = h_sizes[2], nbp = h_sizes[3], n_tiles = h_sizes[4];
   if (ra + 1 > kRowMask || rb + 1 > INT_MAX) return LAMB_GPU_OK;  // panel rows beyond the entry format: not run
-  // ---- digit panels (one zero row at the end of each plane for padding reads) ----
+  // ---- digit panels ----
   const int64_t plane_a = ((ra + 1) * 128 + 255) & ~255ll, plane_b = ((rb + 1) * 64 + 255) & ~255ll;
   int8_t *pan_a = nullptr, *pan_b = nullptr;
   LAMB_TRY(scratch(ctx, kScrPlaneA, plane_a * kS, &pan_a));
   LAMB_TRY(scratch(ctx, kScrPlaneB, plane_b * kS, &pan_b));
-  LAMB_CUDA(ctx, cudaMemsetAsync(pan_a, 0, (size_t)(plane_a * kS), ctx->stream));
-  LAMB_CUDA(ctx, cudaMemsetAsync(pan_b, 0, (size_t)(plane_b * kS), ctx->stream));
-  k_tc_digits_a<<<grid_for(32ll * kDigitWays * A->n_rows, 256), 256, 0, ctx->stream>>>(
-      A->n_rows, A->row_p, A->col, A->off, A->row_bs, A->col_bs, A->data, d_rcl, d_roff, W, bma, wra, basea, mp.rbase,
-      mp.ea, plane_a, pan_a);
+  int4 *pairs_a, *pairs_b;
+  long long *tab_a, *tab_b;
+  LAMB_TRY(m.alloc(&pairs_a, na)); LAMB_TRY(m.alloc(&pairs_b, nbp));
+  const int64_t n_tab = na * kMaxRowAtoms + nbp * kMaxColAtoms;
+  LAMB_TRY(m.alloc(&tab_a, n_tab));
+  tab_b = tab_a + na * kMaxRowAtoms;
+  LAMB_CUDA(ctx, cudaMemsetAsync(tab_a, 0xff, sizeof(long long) * n_tab, ctx->stream));
+  k_tc_pairs<<<grid_for((int64_t)rc.n * W, 64), 64, 0, ctx->stream>>>(rc.n, W, bma, A->col_bs, wra, basea, pba, pairs_a);
   LAMB_LAUNCHED(ctx);
-  k_tc_digits_b<<<grid_for(32ll * kDigitWays * B->n_rows, 256), 256, 0, ctx->stream>>>(
-      B->n_rows, B->row_p, B->col, B->off, B->row_bs, B->col_bs, B->data, d_ccl, d_coff, W, bmb, wrb, baseb, mp.cbase,
-      mp.eb, plane_b, pan_b);
+  k_tc_pairs<<<grid_for((int64_t)cc.n * W, 64), 64, 0, ctx->stream>>>(cc.n, W, bmb, B->row_bs, wrb, baseb, pbb, pairs_b);
+  LAMB_LAUNCHED(ctx);
+  k_tc_pair_blocks<true><<<grid_for(32ll * A->n_rows, 256), 256, 0, ctx->stream>>>(
+      A->n_rows, W, A->row_p, A->col, A->off, rc.of, rc.idx, bma, wra, pba, tab_a);
+  LAMB_LAUNCHED(ctx);
+  k_tc_pair_blocks<false><<<grid_for(32ll * B->n_rows, 256), 256, 0, ctx->stream>>>(
+      B->n_rows, W, B->row_p, B->col, B->off, cc.of, cc.idx, bmb, wrb, pbb, tab_b);
+  LAMB_LAUNCHED(ctx);
+  auto warps = [](int64_t n) { return 32 * ((n + kDigitPairs - 1) / kDigitPairs); };
+  k_tc_digits<true><<<grid_for(warps(na), 128), 128, 0, ctx->stream>>>(na, pairs_a, tab_a, rc.geo, d_rc_exp, A->data,
+                                                                       plane_a, pan_a);
+  LAMB_LAUNCHED(ctx);
+  k_tc_digits<false><<<grid_for(warps(nbp), 128), 128, 0, ctx->stream>>>(nbp, pairs_b, tab_b, cc.geo, d_cc_exp, B->data,
+                                                                         plane_b, pan_b);
   LAMB_LAUNCHED(ctx);
   // ---- tile list, C block lists, inner lists ----
   int2* tiles;
@@ -1333,7 +1434,7 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   k_tc_tile_stats<<<grid_for(n_tiles, 256), 256, 0, ctx->stream>>>(n_tiles, krows, d_stats);
   LAMB_LAUNCHED(ctx);
   LAMB_CUDA(ctx, cudaMemcpyAsync(d_stats + 2, ebase + n_tiles, sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->stream));
-  auto* h_stats = reinterpret_cast<volatile unsigned long long*>(ctx->pin + kPinTc + 3);
+  auto* h_stats = reinterpret_cast<volatile unsigned long long*>(ctx->pin + kPinTc + 5);
   LAMB_CUDA(ctx, cudaMemcpyAsync((void*)h_stats, d_stats, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   const int64_t max_rows = (int64_t)h_stats[0], n_ent = (int64_t)h_stats[2];
@@ -1354,14 +1455,14 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   g.pan_a = pan_a; g.plane_a = plane_a; g.pan_b = pan_b; g.plane_b = plane_b;
   g.cc_first = cc.first;
   g.blist = blist; g.lbase = lbase; g.c_data = C->data; g.c_nrm = c_nrm; g.err = d_err;
-  g.rc_exp = d_rc_exp; g.rc_row = rc.desc; g.cc_exp = d_cc_exp; g.cc_ab = cc.desc;
+  g.rc_exp = d_rc_exp; g.rc_row = rc.geo; g.cc_exp = d_cc_exp; g.cc_ab = cc.cab;
   LAMB_CUDA(ctx, cudaFuncSetAttribute(k_tc_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const int grid = (int)std::min<int64_t>(n_tiles, sms);
   k_tc_tiles<<<grid, kTileThreads, kSmemBytes, ctx->stream>>>(g);
   LAMB_LAUNCHED(ctx);
-  auto* p_err = reinterpret_cast<volatile int*>(ctx->pin + kPinTc + 7);
+  auto* p_err = reinterpret_cast<volatile int*>(ctx->pin + kPinTc + 8);
   LAMB_CUDA(ctx, cudaMemcpyAsync((void*)p_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   const int h_err = *p_err;

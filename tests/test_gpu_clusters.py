@@ -92,3 +92,15 @@ def test_inner_runs(gpu_ctx, runs, sizes):
     a = _matrix(rng, rows, inner, pa)
     b = _matrix(rng, inner, cols, np.ones((n, 2), bool))
     _check(gpu_ctx, a, b, None)
+
+
+@pytest.mark.parametrize("ea,eb", [(600, -600), (-1005, 1000), (-1005, 5)])
+def test_wide_exponents(gpu_ctx, ea, eb):
+    """Row and column scales beyond what a single exact factor covers."""
+    rng = np.random.default_rng(7)
+    s = np.array([13, 5, 5])
+    a, b = _band(rng, 60, 60, s, s), _band(rng, 60, 60, s, s)
+    for m, e in ((a, ea), (b, eb)):
+        for sec in m.sectors:
+            sec.data[:] = np.ldexp(sec.data, e)
+    _check(gpu_ctx, a, b, _positions(rng, 60, "line"))
