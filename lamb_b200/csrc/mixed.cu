@@ -48,13 +48,13 @@ constexpr int64_t kLevelInnerMax7 = (int64_t)INT_MAX / (7 * 64 * 64);
 __device__ __forceinline__ int pad4(int x) { return (x + 3) & ~3; }
 
 // ---- scales ----------------------------------------------------------------------------
-// Row exponents of A: one CTA per block row, its warps taking every 8th
-// block of the row (memory parallelism across the row's blocks).  For
+// Row exponents of A: one CTA per block row, its warps taking every 8th (32nd
+// where rows are few) block of the row (memory parallelism across the row's blocks).  For
 // bi <= 32 lane l keeps the running max of element row l % bi over the
 // columns l / bi, l / bi + 32 / bi, ... of its blocks; all lanes of one
 // element row then merge through a shared-memory atomic max (non-negative
 // doubles order like their bit patterns).  Larger blocks merge every element.
-__global__ void k_row_exp(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
+__global__ void __launch_bounds__(1024) k_row_exp(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
                           const int64_t* __restrict__ off, const int8_t* __restrict__ row_bs,
                           const int8_t* __restrict__ col_bs, const double* __restrict__ d,
                           const int64_t* __restrict__ ebase, int* __restrict__ ea) {
@@ -94,16 +94,16 @@ __global__ void k_row_exp(int32_t n_rows, const int64_t* __restrict__ row_p, con
   }
 }
 
-// Column exponents of B: one CTA per block row, its warps taking every 8th
-// block of the row.  For bj <= 32 lane l keeps the max of element column
+// Column exponents of B: one CTA per block row, its warps taking every 8th or
+// 32nd block of the row.  For bj <= 32 lane l keeps the max of element column
 // l % bj over the rows l / bj, l / bj + 32 / bj, ...; the lanes of one
 // column merge through a shared-memory atomic max, then one global atomic
 // max per block column element.
-__global__ void k_col_exp(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
+__global__ void __launch_bounds__(1024) k_col_exp(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
                           const int64_t* __restrict__ off, const int8_t* __restrict__ row_bs,
                           const int8_t* __restrict__ col_bs, const double* __restrict__ d,
                           const int64_t* __restrict__ ebase, int* __restrict__ eb) {
-  __shared__ unsigned long long cm[8][128];
+  __shared__ unsigned long long cm[32][128];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5, nwl = blockDim.x >> 5;
   for (int64_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
     const int bk = row_bs[r];
@@ -447,15 +447,18 @@ int32_t build_slices(Ctx* ctx, const DevMatrix* A, const DevMatrix* B, int s, Mi
   LAMB_CUDA(ctx, cudaMemcpyAsync(mp->cbase, cbv.data(), sizeof(int64_t) * cbv.size(), cudaMemcpyHostToDevice, ctx->stream));
   LAMB_TRY(dalloc(ctx, &mp->ea, std::max<int64_t>(ra.back(), 1)));
   LAMB_TRY(dalloc(ctx, &mp->eb, std::max<int64_t>(cbv.back(), 1)));
+  // Few rows leave the SMs short of loads in flight with eight warps a row (288
+  // dense rows: 62 and 77 -> 29 and 33 us with 32).
+  auto exp_threads = [](int32_t rows) { return rows < 8 * 148 ? 1024 : kThreads; };
   // eb starts at 0x80808080 (byte fill), below any frexp exponent, for the atomic max
   LAMB_CUDA(ctx, cudaMemsetAsync(mp->eb, 0x80, sizeof(int) * std::max<int64_t>(cbv.back(), 1), ctx->stream));
   if (A->nnz) {
-    k_row_exp<<<grid_for((int64_t)A->n_rows * kThreads), kThreads, 0, ctx->stream>>>(
+    k_row_exp<<<grid_for((int64_t)A->n_rows * kThreads), exp_threads(A->n_rows), 0, ctx->stream>>>(
         A->n_rows, A->row_p, A->col, A->off, A->row_bs, A->col_bs, A->data, mp->rbase, mp->ea);
     LAMB_LAUNCHED(ctx);
   }
   if (B->nnz) {
-    k_col_exp<<<grid_for((int64_t)B->n_rows * kThreads), kThreads, 0, ctx->stream>>>(
+    k_col_exp<<<grid_for((int64_t)B->n_rows * kThreads), exp_threads(B->n_rows), 0, ctx->stream>>>(
         B->n_rows, B->row_p, B->col, B->off, B->row_bs, B->col_bs, B->data, mp->cbase, mp->eb);
     LAMB_LAUNCHED(ctx);
   }
