@@ -366,7 +366,7 @@ def run_ours(args):
     flops = stats[-1]["flops"]
     value = flops * args.steps * world / (ms_max * 1e-3) / 1e9
     ms_num = statistics.mean(s["ms_numeric"] for s in stats)
-    ms_kern = statistics.mean(s["ms_kernel"] for s in stats)  # the k_stacked launches alone
+    ms_kern = statistics.mean(s["ms_kernel"] for s in stats)  # the product kernel (k_panel_tiles) alone
     ms_tot = statistics.mean(s["ms_total"] for s in stats)
     c_host = dc.download()
     alg_bytes = algorithmic_bytes(a, b, c_host)
@@ -433,15 +433,15 @@ def run_ours(args):
             "setup": {"path": "plain FP64 (DMMA)",
                       "row_order": "pattern (Cuthill-McKee)" if args.no_positions else "Morton (atom coordinates)",
                       "l2": "inputs 2x1.9 GB exceed L2; no flush", "parallelism": f"replicas x{world}"},
-            "roofline": {"bound": "tensor", "kernel": "k_stacked", "achieved": achieved_tf,
+            "roofline": {"bound": "tensor", "kernel": "k_panel_tiles", "achieved": achieved_tf,
                          "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved_tf / fp64_peak,
                          "peak_source": "FP64 DMMA probe measured on this GPU in this run",
-                         "traffic": committed_traffic("k_stacked", wl.name),
-                         "traffic_scope": "DRAM bytes of one multiply's k_stacked launches (all row chunks), "
-                                          "scaled from the committed small-case capture; null when none",
+                         "traffic": committed_traffic("k_panel_tiles", wl.name),
+                         "traffic_scope": "DRAM bytes of one multiply's tile-kernel launch, scaled by block products "
+                                          "from the committed small-case capture; null when none",
                          "flops_per_multiply": flops, "ms_per_multiply": ms_kern,
-                         "timing": "CUDA events around each row chunk's k_stacked launch, summed per multiply "
-                                   "(the chunks' stack fills excluded); numeric phase with fills: "
+                         "timing": "CUDA events around the product kernel's launches, summed per multiply; "
+                                   "numeric phase with the panels' packing: "
                                    f"{ms_num:.2f} ms"},
             "roofline_hbm": {"bound": "hbm", "achieved": alg_bytes / (ms_tot * 1e-3) / 1e9,
                              "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
