@@ -43,14 +43,13 @@
 //   warp 7     expands the tiles' inner lists (runs of panel rows) into the 32
 //              (A row, B row) pairs of every stage, up to kRing stages ahead
 //              of the producers;
-//   warps 8-15 epilogue: tensor memory -> FP64 staging tile in shared
-//              memory (the six levels of a column recombined exactly in two
-//              int64 sums), then column scaling and per-row partial sums of
-//              squares per column atom; every C block of the tile copied out
-//              in its storage order (contiguous stores, one warp a block)
-//              and its norm summed from the row partials.  The tile's block
-//              list (built before the kernel) and exponents are loaded one
-//              tile ahead into registers.
+//   warps 8-15 epilogue, two threads a tile row: tensor memory -> FP64 staging
+//              tile in shared memory (the six levels of a column recombined
+//              exactly in two int64 sums); then every thread writes its row,
+//              scaled, into the C blocks of its row atom and keeps the sums
+//              of squares per column atom, from which the block norms are
+//              summed.  The tile's block list (built before the kernel) and
+//              exponents are loaded one tile ahead into registers.
 // What bounds it: the MMAs of a stage take ~665 clocks (the tensor pipe and its
 // operand reads from shared memory, ~590), the copies of a stage ~350 of the
 // producers' time.  With three stages the MMAs waited a third of the time for
