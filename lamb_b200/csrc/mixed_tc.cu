@@ -670,6 +670,11 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
 namespace lamb {
 namespace tc {
 
+// Warps a block row in the kernels below that list blocks: with one, 288 dense
+// rows leave most of the GPU idle (bitmaps, pair blocks, tile flags and tile
+// lists together 98 -> 65 us there; no change at 4,608 rows of 380 blocks).
+constexpr int kRowWays = 8;
+
 // Bitmap bit (cluster, inner atom k): A (by_row): cluster of row r, k = column;
 // B (!by_row): cluster of column c, k = row r.  The lanes whose bits share a word
 // join them, and write only what is missing: dense rows hit the same words over
@@ -677,8 +682,9 @@ namespace tc {
 __global__ void k_tc_bitmap(int32_t n_rows, const int64_t* __restrict__ row_p, const int32_t* __restrict__ col,
                             const int32_t* __restrict__ clus, int by_row, int32_t W, uint32_t* bm) {
   const int lane = threadIdx.x & 31;
-  for (int64_t r = global_warp(); r < n_rows; r += grid_warps())
-    for (int64_t b = row_p[r] + lane; b < row_p[r + 1]; b += 32) {
+  for (int64_t gw = global_warp(); gw < (int64_t)n_rows * kRowWays; gw += grid_warps()) {
+    const int64_t r = gw / kRowWays;
+    for (int64_t b = row_p[r] + 32 * (gw % kRowWays) + lane; b < row_p[r + 1]; b += 32 * kRowWays) {
       const int c = col[b];
       const int cl = by_row ? clus[r] : clus[c];
       const int k = by_row ? c : (int)r;
@@ -687,6 +693,7 @@ __global__ void k_tc_bitmap(int32_t n_rows, const int64_t* __restrict__ row_p, c
       const uint32_t bits = __reduce_or_sync(peers, 1u << (k & 31));
       if (lane == __ffs(peers) - 1 && (__ldcg(&bm[word]) & bits) != bits) atomicOr(&bm[word], bits);
     }
+  }
 }
 
 // Panel rows and pairs (cluster, inner atom) of every cluster before each bitmap word, and their totals.
@@ -768,13 +775,15 @@ __global__ void k_tc_pair_blocks(int32_t n_rows, int32_t W, const int64_t* __res
                                  const int64_t* __restrict__ pair_base, long long* __restrict__ tab) {
   constexpr int per = A_SIDE ? kMaxRowAtoms : kMaxColAtoms;
   const int lane = threadIdx.x & 31;
-  for (int64_t i = global_warp(); i < n_rows; i += grid_warps())
-    for (int64_t b = row_p[i] + lane; b < row_p[i + 1]; b += 32) {
+  for (int64_t gw = global_warp(); gw < (int64_t)n_rows * kRowWays; gw += grid_warps()) {
+    const int64_t i = gw / kRowWays;
+    for (int64_t b = row_p[i] + 32 * (gw % kRowWays) + lane; b < row_p[i + 1]; b += 32 * kRowWays) {
       const int j = col[b], a = A_SIDE ? (int)i : j, k = A_SIDE ? j : (int)i, c = clus[a];
       const int64_t x = (int64_t)c * W + (k >> 5);
       const int64_t pair = pair_base[c] + before[x].y + __popc(bm[x] & ((1u << (k & 31)) - 1u));
       tab[pair * per + idx[a]] = off[b];
     }
+  }
 }
 
 // x * 2^-e: an exact power-of-two multiply where 2^-e is a normal double
@@ -905,9 +914,11 @@ __global__ void k_tc_tile_flags(int32_t n_rows, const int64_t* __restrict__ row_
                                 const int32_t* __restrict__ rcl, const int32_t* __restrict__ ccl, int32_t n_cc,
                                 int64_t* __restrict__ flag) {
   const int lane = threadIdx.x & 31;
-  for (int64_t i = global_warp(); i < n_rows; i += grid_warps()) {
+  for (int64_t gw = global_warp(); gw < (int64_t)n_rows * kRowWays; gw += grid_warps()) {
+    const int64_t i = gw / kRowWays;
     const int I = rcl[i];
-    for (int64_t b = row_p[i] + lane; b < row_p[i + 1]; b += 32) flag[tile_slot(I, ccl[col[b]], n_cc)] = 1;
+    for (int64_t b = row_p[i] + 32 * (gw % kRowWays) + lane; b < row_p[i + 1]; b += 32 * kRowWays)
+      flag[tile_slot(I, ccl[col[b]], n_cc)] = 1;
   }
 }
 
@@ -934,10 +945,11 @@ __global__ void k_tc_tile_blocks(int32_t n_rows, const int64_t* __restrict__ row
                                  const int64_t* __restrict__ pos, int64_t* __restrict__ cnt,
                                  const int64_t* __restrict__ lbase, int4* __restrict__ blist) {
   const int lane = threadIdx.x & 31;
-  for (int64_t i = global_warp(); i < n_rows; i += grid_warps()) {
+  for (int64_t gw = global_warp(); gw < (int64_t)n_rows * kRowWays; gw += grid_warps()) {
+    const int64_t i = gw / kRowWays;
     const int I = rcl[i];
     const int geo_r = roff[i] | ((int)row_bs[i] << 7) | (ratom[i] << 14);
-    for (int64_t b = row_p[i] + lane; b < row_p[i + 1]; b += 32) {
+    for (int64_t b = row_p[i] + 32 * (gw % kRowWays) + lane; b < row_p[i + 1]; b += 32 * kRowWays) {
       const int j = col[b];
       const int64_t t = pos[tile_slot(I, ccl[j], n_cc)];
       const int64_t slot = (int64_t)atomicAdd(reinterpret_cast<unsigned long long*>(&cnt[t]), 1ull);
@@ -1345,9 +1357,9 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   int64_t *pba = basea + n_a, *baseb = pba + n_a, *pbb = baseb + n_b;
   uint32_t *bma = reinterpret_cast<uint32_t*>(tpb + n_b), *bmb = bma + (int64_t)rc.n * W;
   LAMB_CUDA(ctx, cudaMemsetAsync(tra, 0, (size_t)zeroed, ctx->stream));
-  k_tc_bitmap<<<grid_for(32ll * A->n_rows, 256), 256, 0, ctx->stream>>>(A->n_rows, A->row_p, A->col, d_rcl, 1, W, bma);
+  k_tc_bitmap<<<grid_for(32ll * kRowWays * A->n_rows, 256), 256, 0, ctx->stream>>>(A->n_rows, A->row_p, A->col, d_rcl, 1, W, bma);
   LAMB_LAUNCHED(ctx);
-  k_tc_bitmap<<<grid_for(32ll * B->n_rows, 256), 256, 0, ctx->stream>>>(B->n_rows, B->row_p, B->col, d_ccl, 0, W, bmb);
+  k_tc_bitmap<<<grid_for(32ll * kRowWays * B->n_rows, 256), 256, 0, ctx->stream>>>(B->n_rows, B->row_p, B->col, d_ccl, 0, W, bmb);
   LAMB_LAUNCHED(ctx);
   k_tc_word_prefix<<<grid_for(32ll * rc.n, 256), 256, 0, ctx->stream>>>(rc.n, W, bma, A->col_bs, wra, tra, tpa);
   LAMB_LAUNCHED(ctx);
@@ -1360,7 +1372,7 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   int64_t *flag, *pos;
   LAMB_TRY(m.alloc(&flag, n_map + 1)); LAMB_TRY(m.alloc(&pos, n_map + 1));
   LAMB_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(int64_t) * (size_t)(n_map + 1), ctx->stream));
-  k_tc_tile_flags<<<grid_for(32ll * C->n_rows, 256), 256, 0, ctx->stream>>>(C->n_rows, C->row_p, C->col, d_rcl, d_ccl,
+  k_tc_tile_flags<<<grid_for(32ll * kRowWays * C->n_rows, 256), 256, 0, ctx->stream>>>(C->n_rows, C->row_p, C->col, d_rcl, d_ccl,
                                                                          cc.n, flag);
   LAMB_LAUNCHED(ctx);
   LAMB_TRY(exclusive_scan_i64(ctx, flag, pos, n_map + 1));
@@ -1388,10 +1400,10 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   LAMB_LAUNCHED(ctx);
   k_tc_pairs<<<grid_for((int64_t)cc.n * W, 64), 64, 0, ctx->stream>>>(cc.n, W, bmb, B->row_bs, wrb, baseb, pbb, pairs_b);
   LAMB_LAUNCHED(ctx);
-  k_tc_pair_blocks<true><<<grid_for(32ll * A->n_rows, 256), 256, 0, ctx->stream>>>(
+  k_tc_pair_blocks<true><<<grid_for(32ll * kRowWays * A->n_rows, 256), 256, 0, ctx->stream>>>(
       A->n_rows, W, A->row_p, A->col, A->off, rc.of, rc.idx, bma, wra, pba, tab_a);
   LAMB_LAUNCHED(ctx);
-  k_tc_pair_blocks<false><<<grid_for(32ll * B->n_rows, 256), 256, 0, ctx->stream>>>(
+  k_tc_pair_blocks<false><<<grid_for(32ll * kRowWays * B->n_rows, 256), 256, 0, ctx->stream>>>(
       B->n_rows, W, B->row_p, B->col, B->off, cc.of, cc.idx, bmb, wrb, pbb, tab_b);
   LAMB_LAUNCHED(ctx);
   auto warps = [](int64_t n) { return 32 * ((n + kDigitPairs - 1) / kDigitPairs); };
@@ -1416,13 +1428,13 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   k_tc_tile_list<<<grid_for(n_map, 256), 256, 0, ctx->stream>>>(n_map, cc.n, flag, pos, tiles);
   LAMB_LAUNCHED(ctx);
   LAMB_CUDA(ctx, cudaMemsetAsync(lcnt, 0, sizeof(int64_t) * (size_t)(n_tiles + 1), ctx->stream));
-  k_tc_tile_blocks<false><<<grid_for(32ll * C->n_rows, 256), 256, 0, ctx->stream>>>(
+  k_tc_tile_blocks<false><<<grid_for(32ll * kRowWays * C->n_rows, 256), 256, 0, ctx->stream>>>(
       C->n_rows, C->row_p, C->col, C->off, C->row_bs, d_rcl, d_roff, d_ratom, d_ccl, d_catom, cc.n, pos, lcnt, nullptr,
       nullptr);
   LAMB_LAUNCHED(ctx);
   LAMB_TRY(exclusive_scan_i64(ctx, lcnt, lbase, n_tiles + 1));
   LAMB_CUDA(ctx, cudaMemsetAsync(lcnt, 0, sizeof(int64_t) * (size_t)(n_tiles + 1), ctx->stream));
-  k_tc_tile_blocks<true><<<grid_for(32ll * C->n_rows, 256), 256, 0, ctx->stream>>>(
+  k_tc_tile_blocks<true><<<grid_for(32ll * kRowWays * C->n_rows, 256), 256, 0, ctx->stream>>>(
       C->n_rows, C->row_p, C->col, C->off, C->row_bs, d_rcl, d_roff, d_ratom, d_ccl, d_catom, cc.n, pos, lcnt, lbase,
       blist);
   LAMB_LAUNCHED(ctx);
