@@ -141,6 +141,7 @@ struct Ctx {
   void* stage[kPinSlots] = {};
   size_t stage_bytes[kPinSlots] = {};
   int* tile_err = nullptr;  // device: set by the panel kernel when one of its bounded waits ran out
+  uint64_t wait_ns = 2000000000ull;  // that bound (LAMB_GPU_WAIT_MS at creation; 0: every wait counts as run out)
 };
 // Words of the pinned buffer.
 constexpr int kPinCount = 0;    // what the symbolic count leaves (CountStat, 5 words)

@@ -763,6 +763,11 @@ int32_t lamb_gpu_ctx_create(int32_t device, lamb_gpu_ctx** out) {
     return make_status(LAMB_LEVEL_MEMORY, LAMB_TYPE_EXTERNAL_ERROR);
   }
   ctx->pin[kPinTileErr] = 0;
+  if (const char* w = std::getenv("LAMB_GPU_WAIT_MS")) {
+    char* end = nullptr;
+    const unsigned long ms = std::strtoul(w, &end, 10);
+    if (end != w && ms <= 2000) ctx->wait_ns = 1000000ull * ms;
+  }
   if (const char* t = std::getenv("LAMB_GPU_TRACE")) {
     ctx->trace = t[0] == '1' || t[0] == '2';
     ctx->trace_host = t[0] == '2';

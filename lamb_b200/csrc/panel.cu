@@ -381,6 +381,7 @@ struct TileArgs {
   const int32_t* seg;  // first item of every super row
   int32_t s0, s1;
   int32_t* head;  // items taken
+  uint64_t wait_ns;  // longest wait for a copy
   int* err;
 };
 
@@ -391,17 +392,22 @@ struct __align__(128) WarpSm {
 constexpr size_t kTileSmem = sizeof(WarpSm) * kTileWarps + 128;
 static_assert(kTileSmem <= 232448, "the tile kernel exceeds the shared memory of one CTA");
 
-// Waits for the phase of the given parity, at most 2 s; then records `code`
-// and stops the CTA.
-__device__ __forceinline__ bool tile_wait(unsigned long long* b, uint32_t parity, int* abort, int* err, int code) {
-  if (bar_try(b, parity)) return true;
+// Waits for the phase of the given parity, at most limit_ns; then records
+// `code` and stops the CTA.  The answer is the whole warp's: lanes that left
+// by themselves would be missing from the shuffles of the others.  A limit of
+// 0 counts every wait as run out, without looking.
+__device__ __forceinline__ bool tile_wait(unsigned long long* b, uint32_t parity, uint64_t limit_ns, int* abort,
+                                          int* err, int code) {
+  if (__all_sync(0xffffffffu, limit_ns != 0 && bar_try(b, parity))) return true;
   const uint64_t t0 = now_ns();
   for (;;) {
-    if (bar_try_sleep(b, parity, 20000u)) return true;
-    if (*(volatile int*)abort) return false;
-    if (now_ns() - t0 > 2000000000ull) {
-      atomicOr(err, code);
-      *(volatile int*)abort = 1;
+    if (__all_sync(0xffffffffu, limit_ns != 0 && bar_try_sleep(b, parity, 20000u))) return true;
+    if (__any_sync(0xffffffffu, *(volatile int*)abort)) return false;
+    if (__any_sync(0xffffffffu, now_ns() - t0 >= limit_ns)) {
+      if ((threadIdx.x & 31) == 0) {
+        atomicOr(err, code);
+        *(volatile int*)abort = 1;
+      }
       return false;
     }
   }
@@ -636,7 +642,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 1) k_panel_tiles(const __grid
       const bool csplit = nsplit;
       have = advance();
       if (have) issue(slot ^ 1);
-      if (!(ok = tile_wait(&ws.full[slot], (ph >> slot) & 1u, abort, p.err, 1))) break;
+      if (!(ok = tile_wait(&ws.full[slot], (ph >> slot) & 1u, p.wait_ns, abort, p.err, 1))) break;
       ph ^= 1u << slot;
       const double* pa = ws.ring[slot][0] + pair;
       const double* ps = ws.ring[slot][0] + single;
@@ -1171,6 +1177,7 @@ int32_t panel_tiles(Ctx* ctx, const PanelPair& p, const DevMatrix* C, const uint
   t.i_bs = p.a.rows_out ? p.a.m->col_bs : p.a.m->row_bs;
   t.nk_max = K.max_atoms;
   t.items = q.items; t.seg = q.count; t.head = q.count + n_sup + 1; t.err = ctx->tile_err;
+  t.wait_ns = ctx->wait_ns;
   const size_t smem = kTileSmem;
   auto kern = filt ? k_panel_tiles<true> : k_panel_tiles<false>;
   LAMB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
