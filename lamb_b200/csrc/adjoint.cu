@@ -284,8 +284,7 @@ int32_t adjoint_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* dC, DevMat
     free_tindex(ctx, ct);
     LAMB_TRY(rc);
   }
-  LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return LAMB_GPU_OK;
+  return finish(ctx);
 }
 
 }  // namespace lamb

@@ -480,8 +480,7 @@ int32_t lamb_gpu_matrix_axpby(lamb_gpu_ctx* c, double alpha, lamb_gpu_matrix x, 
   if (!X || !Y) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "axpby: invalid handle");
   if (X == Y) return scale_shift_impl(ctx, Y, alpha + beta, 0.0);
   int32_t rc = axpby_impl(ctx, alpha, X, beta, Y);
-  if (rc == LAMB_GPU_OK) LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return rc;
+  return rc == LAMB_GPU_OK ? finish(ctx) : rc;
 }
 
 int32_t lamb_gpu_matrix_copy(lamb_gpu_ctx* c, lamb_gpu_matrix x, lamb_gpu_matrix y) {
@@ -489,36 +488,39 @@ int32_t lamb_gpu_matrix_copy(lamb_gpu_ctx* c, lamb_gpu_matrix x, lamb_gpu_matrix
   DevMatrix *X = get_matrix(ctx, x), *Y = get_matrix(ctx, y);
   if (!X || !Y) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "copy: invalid handle");
   LAMB_TRY(copy_impl(ctx, X, Y));
-  LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return LAMB_GPU_OK;
+  return finish(ctx);
 }
 
 int32_t lamb_gpu_matrix_trace(lamb_gpu_ctx* c, lamb_gpu_matrix x, double* tr) {
   CTX_OR_FAIL(c);
   DevMatrix* X = get_matrix(ctx, x);
   if (!X || !tr) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "trace: invalid argument");
-  return trace_impl(ctx, X, tr);
+  LAMB_TRY(trace_impl(ctx, X, tr));
+  return finish(ctx);
 }
 
 int32_t lamb_gpu_matrix_trace_product(lamb_gpu_ctx* c, lamb_gpu_matrix x, lamb_gpu_matrix y, double* tr) {
   CTX_OR_FAIL(c);
   DevMatrix *X = get_matrix(ctx, x), *Y = get_matrix(ctx, y);
   if (!X || !Y || !tr) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "trace_product: invalid argument");
-  return trace_product_impl(ctx, X, Y, tr);
+  LAMB_TRY(trace_product_impl(ctx, X, Y, tr));
+  return finish(ctx);
 }
 
 int32_t lamb_gpu_matrix_frobenius(lamb_gpu_ctx* c, lamb_gpu_matrix x, double* norm) {
   CTX_OR_FAIL(c);
   DevMatrix* X = get_matrix(ctx, x);
   if (!X || !norm) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "frobenius: invalid argument");
-  return frobenius_impl(ctx, X, norm);
+  LAMB_TRY(frobenius_impl(ctx, X, norm));
+  return finish(ctx);
 }
 
 int32_t lamb_gpu_matrix_diff_frobenius(lamb_gpu_ctx* c, lamb_gpu_matrix x, lamb_gpu_matrix y, double* norm) {
   CTX_OR_FAIL(c);
   DevMatrix *X = get_matrix(ctx, x), *Y = get_matrix(ctx, y);
   if (!X || !Y || !norm) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "diff_frobenius: invalid argument");
-  return diff_frobenius_impl(ctx, X, Y, norm);
+  LAMB_TRY(diff_frobenius_impl(ctx, X, Y, norm));
+  return finish(ctx);
 }
 
 int32_t lamb_gpu_matrix_scale_shift(lamb_gpu_ctx* c, lamb_gpu_matrix x, double alpha, double shift) {
@@ -526,8 +528,7 @@ int32_t lamb_gpu_matrix_scale_shift(lamb_gpu_ctx* c, lamb_gpu_matrix x, double a
   DevMatrix* X = get_matrix(ctx, x);
   if (!X) return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "scale_shift: invalid handle");
   LAMB_TRY(scale_shift_impl(ctx, X, alpha, shift));
-  LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return LAMB_GPU_OK;
+  return finish(ctx);
 }
 
 }  // extern "C"

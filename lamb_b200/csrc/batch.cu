@@ -420,6 +420,7 @@ static int32_t batch_run(Batch* B, uint32_t flags, lamb_gpu_mult_stats* stats) {
   LAMB_CUDA(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
   LAMB_CUDA(ctx, cudaEventSynchronize(ctx->ev[3]));
   LAMB_TRY(settle(ctx));
+  LAMB_TRY(check_tiles(ctx));  // of an operand: the batch itself runs on stacks
   if (full) {
     for (DevMatrix* C : B->c) after += C->nnz;
     record_gens(B);

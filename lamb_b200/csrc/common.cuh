@@ -155,8 +155,12 @@ constexpr int kPinWords = 64;
 struct NormRange {
   unsigned long long not_min, max;
 };
-// Reports (once) that a panel product stopped; the stream has been waited for.
+// Reports that a panel product stopped; the stream has been waited for.  The
+// flag stays until one caller has been told: only calls that return data, or a
+// product made from it, look (not settle(), whose callers may drop its status).
 int32_t check_tiles(Ctx* ctx);
+// Waits for the stream, then check_tiles: the end of every call that returns data.
+int32_t finish(Ctx* ctx);
 
 // Completes a pending result filter (waits for its counts and updates the
 // matrix's host metadata).  Every entry point reaches it through get_matrix.

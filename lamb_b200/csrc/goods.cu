@@ -203,8 +203,7 @@ int32_t lamb_gpu_goods_pack(lamb_gpu_ctx* c, lamb_gpu_matrix h, int32_t sector, 
   const int32_t rc = body();
   if (!here) dfree(ctx, msg);
   LAMB_TRY(rc);
-  LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return LAMB_GPU_OK;
+  return finish(ctx);
 }
 
 int32_t lamb_gpu_goods_unpack(lamb_gpu_ctx* c, const int64_t* index, int64_t index_words, const double* data,

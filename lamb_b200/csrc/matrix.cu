@@ -92,6 +92,11 @@ void trace_mark(Ctx* ctx, const char* what) {
   ctx->trace_t = now;
 }
 
+int32_t finish(Ctx* ctx) {
+  LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  return check_tiles(ctx);
+}
+
 int32_t check_tiles(Ctx* ctx) {
   const int code = (int)*(volatile int*)&ctx->pin[kPinTileErr];
   if (!code) return LAMB_GPU_OK;
@@ -111,7 +116,7 @@ int32_t settle(Ctx* ctx) {
   int64_t tot = 0;
   for (int64_t x : m->sec_nblk) tot += x;
   m->nnz = tot;
-  return check_tiles(ctx);
+  return LAMB_GPU_OK;
 }
 
 DevMatrix* find_matrix(Ctx* ctx, lamb_gpu_matrix h) {
@@ -791,6 +796,7 @@ int32_t lamb_gpu_ctx_destroy(lamb_gpu_ctx* c) {
   ctx->mats.clear();
   release_scratch(ctx);
   cudaStreamSynchronize(ctx->stream);
+  const int32_t rc = check_tiles(ctx);  // the last call that can tell
   for (auto& ev : ctx->ev) cudaEventDestroy(ev);
   for (auto& ev : ctx->chunk_ev) cudaEventDestroy(ev);
   for (auto& row : ctx->kern_ev)
@@ -803,7 +809,7 @@ int32_t lamb_gpu_ctx_destroy(lamb_gpu_ctx* c) {
   cudaFree(ctx->tile_err);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
-  return LAMB_GPU_OK;
+  return rc;
 }
 
 int32_t lamb_gpu_last_error(const lamb_gpu_ctx* c, char* msg, int32_t len) {
@@ -826,8 +832,7 @@ int32_t lamb_gpu_ctx_get_stream(const lamb_gpu_ctx* c, void** stream) {
 int32_t lamb_gpu_ctx_synchronize(lamb_gpu_ctx* c) {
   auto* ctx = reinterpret_cast<Ctx*>(c);
   if (!ctx) return make_status(LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS);
-  LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  return check_tiles(ctx);
+  return finish(ctx);
 }
 
 int32_t lamb_gpu_matrix_upload(lamb_gpu_ctx* c, const lamb_c_sector* sec, int32_t n_sec, lamb_gpu_matrix* handle) {

@@ -434,6 +434,13 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     LAMB_CUDA(ctx, cudaMemcpyAsync(h_cnt, c_cnt, sizeof(int64_t) * 4 * n_rows, cudaMemcpyDeviceToHost, ctx->stream));
     LAMB_CUDA(ctx, cudaMemcpyAsync(ctx->pin + kPinCount, d_stat, sizeof(CountStat), cudaMemcpyDeviceToHost, ctx->stream));
     LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    // an operand may be the result of an asynchronous product that stopped
+    const int32_t rc = check_tiles(ctx);
+    if (rc != LAMB_GPU_OK) {
+      dfree(ctx, c_cnt);
+      dfree(ctx, d_stat);
+      return rc;
+    }
   }
   if (n_rows) {
     const CountStat& h = *reinterpret_cast<const CountStat*>(ctx->pin + kPinCount);
