@@ -36,8 +36,8 @@
 // Kernel roles (one CTA of 512 threads per SM, persistent over the tiles):
 //   warps 0-5  producers: gather the tile's K rows, 32 per pipeline stage
 //              (four warps the A chunks, two warps the B chunks);
-//   warp 6     allocates the tensor memory (6 levels x 64 columns in 512) and
-//              from one lane issues nine MMAs (M=128, K=32, N=64..256) per
+//   warp 6     allocates the tensor memory (6 levels x 64 columns in 512); one
+//              of its threads issues nine MMAs (M=128, K=32, N=64..256) per
 //              stage, one per A digit plane and run of up to four B digit
 //              planes;
 //   warp 7     expands the tiles' inner lists (runs of panel rows) into the 32
@@ -62,7 +62,9 @@
 // by a warp (5.9), eight columns loaded ahead of their stores (6.3).
 // Every wait on an mbarrier is bounded (2 s of %globaltimer); on a timeout
 // the kernel records an error code, every role stops, and the host returns
-// an error status.
+// an error status.  The roles stop by whole warps (a wait answers for its warp),
+// the epilogue by all of its warps at one vote a tile: whoever left alone would
+// be missing from the barriers of the others, which have no limit.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -181,18 +183,25 @@ __device__ __noinline__ double scale_wide(double x, int e) { return ldexp(x, e);
 // 2^e for -1022 <= e <= 1023, exactly.
 __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 // Waits until the phase with the given parity has completed; gives up after
-// 2 s (or when another role aborted), recording `code`.  The waiting thread
-// sleeps between checks, leaving the issue slots to the other warps of its
-// SM sub-partition.
+// 2 s (or when another role aborted), recording `code`.  The waiting threads
+// sleep between checks, leaving the issue slots to the other warps of their SM
+// sub-partition.  Called by a whole warp, and then the answer is the same for
+// every lane, or (ALONE) with an answer for the calling thread only.
+constexpr uint64_t kWaitNs = 2000000000ull;
+template <bool ALONE = false>
 __device__ __forceinline__ bool bar_wait(unsigned long long* b, uint32_t parity, TileSmem* sm, int* err, int code) {
-  if (bar_try(b, parity)) return true;
+  auto all = [](bool x) { return ALONE ? x : (bool)__all_sync(0xffffffffu, x); };
+  auto any = [](bool x) { return ALONE ? x : (bool)__any_sync(0xffffffffu, x); };
+  if (all(bar_try(b, parity))) return true;
   const uint64_t t0 = now_ns();
   for (;;) {
-    if (bar_try_sleep(b, parity, 200000u)) return true;
-    if (*(volatile int*)&sm->abort) return false;
-    if (now_ns() - t0 > 2000000000ull) {
-      atomicOr(err, code);
-      *(volatile int*)&sm->abort = 1;
+    if (all(bar_try_sleep(b, parity, 200000u))) return true;
+    if (any(*(volatile int*)&sm->abort)) return false;
+    if (any(now_ns() - t0 > kWaitNs)) {
+      if (ALONE || (threadIdx.x & 31) == 0) {
+        atomicOr(err, code);
+        *(volatile int*)&sm->abort = 1;
+      }
       return false;
     }
   }
@@ -320,19 +329,23 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
     // 0..255 are A (row u / 8, chunk u % 8), 256..383 are B (row v / 4,
     // chunk v % 4): consecutive lanes copy consecutive chunks of one panel
     // row, so a warp reads whole 128-byte (A) or 64-byte (B) rows.
+    // A lane whose wait ran out copies nothing more and leaves with its warp at
+    // the vote that every stage has anyway (the rows are read before lane 0
+    // gives them back): a vote at each wait cost 1 % of the mixed multiply.
+    bool go = true;
     for (int64_t gs = 0;; ++gs) {
       const int ring = (int)(gs % kRing), stg = (int)(gs % kStages);
-      if (!bar_wait(&sm->bar_row_full[ring], (uint32_t)((gs / kRing) & 1), sm, g.err, kErrTimeoutRows)) break;
+      go = go && bar_wait<true>(&sm->bar_row_full[ring], (uint32_t)((gs / kRing) & 1), sm, g.err, kErrTimeoutRows);
       int2 prow[kUnits / kProducers];
 #pragma unroll
       for (int i = 0; i < kUnits / kProducers; ++i) {
         const int u = pt + kProducers * i;
         prow[i] = sm->rows[ring][u < 256 ? (u >> 3) : ((u - 256) >> 2)];
       }
-      if (prow[0].x == kEndRow) break;
-      __syncwarp();
+      if (!__all_sync(0xffffffffu, go && prow[0].x != kEndRow)) break;
       if (lane == 0) bar_arrive(&sm->bar_row_empty[ring]);
-      if (!bar_wait(&sm->bar_empty[stg], (uint32_t)(((gs / kStages) & 1) ^ 1), sm, g.err, kErrTimeoutEmpty)) break;
+      go = bar_wait<true>(&sm->bar_empty[stg], (uint32_t)(((gs / kStages) & 1) ^ 1), sm, g.err, kErrTimeoutEmpty);
+      if (!go) continue;
       const uint32_t sa = smem_u32(stages + (size_t)stg * kStageBytes);
       const uint32_t sb = sa + kStageA;
 #pragma unroll
@@ -355,6 +368,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
       }
       cp_arrive(&sm->bar_full[stg]);
     }
+    // copies that no stage waited for (after an abort) land before the CTA ends
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp >= kEpiWarp0) {
     // ================= epilogue =================
     const int ew = warp & 3;        // tensor-memory lane quarter (warp id mod 4)
@@ -431,7 +446,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
       ri = nx_ri;
       wide = publish();
     }
-    for (int64_t t = blockIdx.x; t < n_tiles && !sm->abort; t += gridDim.x, ++local) {
+    for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++local) {
       const bool has_next = t + gridDim.x < n_tiles;
       // ---- accumulators: tensor memory -> staging tile, 16 columns a round
       // (a rolled loop: the epilogue's code stays small next to the other
@@ -442,11 +457,11 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
       // by the 2^52 + 2^51 bias.  The row's power of two is folded into w_2
       // and w_5 (exact: |er| <= kExactExp).  Tensor memory is released as
       // soon as the tile is staged: the next tile's MMAs wait for nothing else. ----
-      if (!bar_wait(&sm->bar_tmem_full, (uint32_t)(local & 1), sm, g.err, kErrTimeoutTmemFull)) break;
-      tc_fence_after();
+      const bool ok = bar_wait(&sm->bar_tmem_full, (uint32_t)(local & 1), sm, g.err, kErrTimeoutTmemFull);
       double* row = sm->stg + et * kN;
       const int sw = et & 15;
-      {
+      if (ok) {
+        tc_fence_after();
         const double rs = wide ? 1.0 : pow2(er);
         const double w2 = kLevelW[2] * rs, w5 = kLevelW[5] * rs;
         const uint32_t lane_base = tmem + ((uint32_t)(32 * ew) << 16);
@@ -471,7 +486,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
         prefetch();
         bounds(t + 2 * (int64_t)gridDim.x);
       }
-      named_sync(2, kEpiThreads);  // both halves of every row are staged
+      // both halves of every row are staged, or all leave
+      if (named_sync_or(2, kEpiThreads, !ok)) break;
       // ---- write-out: each thread writes its tile row into the C blocks of
       // its row atom, one column atom after the other (those that start in its
       // half of the columns; a block's column is
@@ -552,7 +568,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
       ++gs;
     };
     bounds(blockIdx.x);
-    for (int64_t t = blockIdx.x; ok && t < n_tiles && !*(volatile int*)&sm->abort; t += gridDim.x) {
+    for (int64_t t = blockIdx.x; ok && t < n_tiles; t += gridDim.x) {
       const int n = (int)nb_cnt, K = nb_k;
       const uint2* __restrict__ ent = g.ent + nb_base;
       const int nst = K > 0 ? (K + kK - 1) / kK : 1;
@@ -605,22 +621,23 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
       }
     }
   } else {
-    // ================= MMA issuer (lane 0) =================
-    int64_t gs = 0, local_mma = 0;
-    bool ok = true;
-    int next_k = (int64_t)blockIdx.x < n_tiles ? g.krows[blockIdx.x] : 0;  // K rows, loaded one tile ahead
-    for (int64_t t = blockIdx.x; ok && t < n_tiles && !*(volatile int*)&sm->abort; t += gridDim.x, ++local_mma) {
-      const int K = next_k;
-      next_k = t + gridDim.x < n_tiles ? g.krows[t + gridDim.x] : 0;
-      const int nst = K > 0 ? (K + kK - 1) / kK : 1;
-      // tensor memory is free once the epilogue has read the previous tile
-      if (!bar_wait(&sm->bar_tmem_empty, (uint32_t)((local_mma & 1) ^ 1), sm, g.err, kErrTimeoutTmemEmpty)) break;
-      tc_fence_after();
-      for (int s = 0; s < nst; ++s, ++gs) {
-        const int stg = (int)(gs % kStages);
-        if (!bar_wait(&sm->bar_full[stg], (uint32_t)((gs / kStages) & 1), sm, g.err, kErrTimeoutFull)) { ok = false; break; }
+    // ================= MMA issuer =================
+    if (lane == 0) {
+      int64_t gs = 0, local_mma = 0;
+      bool ok = true;
+      int next_k = (int64_t)blockIdx.x < n_tiles ? g.krows[blockIdx.x] : 0;  // K rows, loaded one tile ahead
+      for (int64_t t = blockIdx.x; ok && t < n_tiles; t += gridDim.x, ++local_mma) {
+        const int K = next_k;
+        next_k = t + gridDim.x < n_tiles ? g.krows[t + gridDim.x] : 0;
+        const int nst = K > 0 ? (K + kK - 1) / kK : 1;
+        // tensor memory is free once the epilogue has read the previous tile
+        if (!bar_wait<true>(&sm->bar_tmem_empty, (uint32_t)((local_mma & 1) ^ 1), sm, g.err, kErrTimeoutTmemEmpty)) break;
         tc_fence_after();
-        if (lane == 0) {
+        for (int s = 0; s < nst; ++s, ++gs) {
+          const int stg = (int)(gs % kStages);
+          ok = bar_wait<true>(&sm->bar_full[stg], (uint32_t)((gs / kStages) & 1), sm, g.err, kErrTimeoutFull);
+          if (!ok) break;
+          tc_fence_after();
           fence_async_smem();
           const uint32_t sa = smem_u32(stages + (size_t)stg * kStageBytes);
           const uint32_t sb = sa + kStageA;
@@ -643,16 +660,19 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
           }
           mma_commit(&sm->bar_empty[stg]);
         }
-        __syncwarp();
+        if (ok) mma_commit(&sm->bar_tmem_full);
       }
-      if (!ok) break;
-      if (lane == 0) mma_commit(&sm->bar_tmem_full);
-      __syncwarp();
+      // every MMA issued by this CTA has completed before tensor memory is
+      // released, after an abort too (so this wait does not look at it)
+      mma_commit(&sm->bar_done);
+      const uint64_t t0 = now_ns();
+      while (!bar_try_sleep(&sm->bar_done, 0, 200000u))
+        if (now_ns() - t0 > kWaitNs) {
+          atomicOr(g.err, kErrTimeoutDone);
+          break;
+        }
     }
-    // every MMA issued by this CTA has completed before tensor memory is released
-    if (lane == 0) mma_commit(&sm->bar_done);
     __syncwarp();
-    bar_wait(&sm->bar_done, 0, sm, g.err, kErrTimeoutDone);
   }
   tc_fence_before();
   __syncthreads();
