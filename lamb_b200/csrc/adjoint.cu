@@ -245,7 +245,7 @@ int32_t adjoint_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* dC, DevMat
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "adjoint: outputs must be distinct matrices");
   // Group tiles where they win, as for the multiply: 384 waters (cutoff 6, both
   // products) 4.4 -> 2.8 ms a call, the stack building (1.2 ms) included.
-  bool panel = panel_worth(A, B) && dC->nnz > 0;
+  bool panel = panel_worth(A, B) && dC->nnz > 0 && panel_blocks_ok(A->nnz, B->nnz, dC->nnz);
   std::shared_ptr<GroupTab> cols;
   if (panel) {
     if (!A->h_pos.empty()) LAMB_TRY(ensure_row_order(ctx, A));  // the pattern's own order costs more than it gives here

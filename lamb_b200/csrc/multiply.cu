@@ -1034,7 +1034,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       LAMB_TRY(numeric_mixed(ctx, A, B, C, sym, work, work_c, c_nrm, mp));
     } else {
       // an infinity or NaN would meet the zero rows of absent blocks: such operands take the stacks
-      panel = panel && sym.finite && sym.c_nnz > 0 && sym.c_pre &&
+      panel = panel && sym.finite && sym.c_nnz > 0 && sym.c_pre && panel_blocks_ok(A->nnz, B->nnz, sym.c_nnz) &&
               panel_gain(&pair, *A->rgrp, *A->cgrp, *c_grp, A->h_row_bs, B->h_col_bs, sym.n_ent, ctx->pin + kPinPanel) >=
                   kPanelGain;
       if (panel) LAMB_TRY(numeric_panel(ctx, A, C, sym, &pair, eps, c_nrm, !timed, &panel));

@@ -128,17 +128,17 @@ __global__ void __launch_bounds__(1024) k_panel_scan(const __grid_constant__ Pai
   const SideArgs& s = p.s[blockIdx.x];
   typedef cub::BlockScan<int, 1024> BS;
   __shared__ typename BS::TempStorage ts;
-  int carry = 0;
+  long long carry = 0;  // the host refuses a total beyond 32 bits
   for (int g0 = 0; g0 < s.n_out; g0 += 1024) {
     const int g = g0 + threadIdx.x;
     int e, a;
     BS(ts).ExclusiveSum(g < s.n_out ? s.ptr[g] : 0, e, a);
     __syncthreads();
-    if (g < s.n_out) s.ptr[g] = carry + e;
+    if (g < s.n_out) s.ptr[g] = (int)(carry + e);
     carry += a;
   }
   if (threadIdx.x == 0) {
-    s.ptr[s.n_out] = carry;
+    s.ptr[s.n_out] = (int)carry;
     p.totals[blockIdx.x] = carry;
   }
   if (blockIdx.x == 0) {
@@ -475,7 +475,7 @@ __device__ __forceinline__ void run_rows(double (&acc)[3][3][2], uint32_t m, con
 }
 
 // C block of the tile's atom pair x (row atom x / nb, column atom x % nb): its
-// index, and in *hit whether it is in the pattern.
+// index (32 bits: kPanelMaxBlocks), and in *hit whether it is in the pattern.
 __device__ __forceinline__ int find_block(const TileArgs& p, int a0, int b0, int nb, int x, uint32_t* hit) {
   const int a = x / nb, c = b0 + x - a * nb;
   const int64_t r = a0 + a, w = r * p.c_words + (c >> 5);
@@ -969,7 +969,8 @@ static bool panel_shapes_ok(const std::vector<int8_t>& rows, const std::vector<i
 }
 
 bool panel_worth(const DevMatrix* A, const DevMatrix* B) {
-  return A->n_cols > 0 && (double)A->nnz * B->nnz >= (double)(1 << 19) * A->n_cols &&
+  return A->n_cols > 0 && panel_blocks_ok(A->nnz, B->nnz, 0) &&
+         (double)A->nnz * B->nnz >= (double)(1 << 19) * A->n_cols &&
          panel_shapes_ok(A->h_row_bs, A->h_col_bs, B->h_col_bs);
 }
 
@@ -1058,8 +1059,8 @@ int32_t panel_pack(Ctx* ctx, PanelPair* p, const int64_t* totals, bool filt, boo
   PanelSide* sd[2] = {&p->a, &p->b};
   const int slot[2] = {kScrPlaneA, kScrPlaneB};
   // the panels take at most an eighth of the device's memory (they stay with the context)
-  if ((double)(totals[0] + totals[1]) * p->kstride * kRowBytes > (double)ctx->total_mem / 8 || totals[0] >= INT32_MAX ||
-      totals[1] >= INT32_MAX)
+  if ((double)(totals[0] + totals[1]) * p->kstride * kRowBytes > (double)ctx->total_mem / 8 ||
+      totals[0] > kPanelMaxBlocks || totals[1] > kPanelMaxBlocks)
     return LAMB_GPU_OK;
   for (int k = 0; k < 2; ++k) {
     PanelSide& s = *sd[k];

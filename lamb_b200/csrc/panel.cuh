@@ -1,6 +1,7 @@
 // Panel products: the FP64 block product on group tiles (panel.cu).
 #pragma once
 #include "common.cuh"
+#include "panel_limits.cuh"
 
 namespace lamb {
 

@@ -1,0 +1,17 @@
+// What the group tiles (panel.cu) can hold.  Host C++ only, so that the rules
+// can be checked without a GPU.
+#pragma once
+#include <cstdint>
+
+namespace lamb {
+
+// The tile kernel counts superblocks, tiles and C blocks in 32 bits.  A
+// superblock holds at least one block of its operand and a tile at least one of
+// C, so the block counts bound all three.  Beyond: the stacks, whose work items
+// carry 64-bit offsets.
+constexpr int64_t kPanelMaxBlocks = INT32_MAX;
+inline bool panel_blocks_ok(int64_t a_blocks, int64_t b_blocks, int64_t c_blocks) {
+  return a_blocks <= kPanelMaxBlocks && b_blocks <= kPanelMaxBlocks && c_blocks <= kPanelMaxBlocks;
+}
+
+}  // namespace lamb
