@@ -966,6 +966,10 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
   bool tc_path = mixed && mixed_tc_eligible(A, B) && !(force_sync && force_sync[0] == '1');
   sym.use_scratch = true;
   LAMB_TRY(settle(ctx));
+  auto check_norm_index = [&](bool norms) -> int32_t {
+    if (norm_index_ok(sym.c_nnz, norms)) return LAMB_GPU_OK;
+    return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "more than 2^31 blocks in a C with block norms");
+  };
   auto body = [&]() -> int32_t {
     trace_mark(ctx, "multiply: start");
     LAMB_TRY(check_compatible(ctx, A, B));
@@ -978,6 +982,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       LAMB_TRY(build_slices(ctx, A, B, slices, &mp, true));
       sym.pattern_only = true;
       LAMB_TRY(symbolic_phase(ctx, A, B, C, eps, filt_p, false, nullptr, &sym));
+      LAMB_TRY(check_norm_index(true));
       LAMB_TRY(dalloc(ctx, &c_nrm, std::max<int64_t>(sym.c_nnz, 1)));
       if (timed) LAMB_CUDA(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
       trace_mark(ctx, "symbolic (pattern)");
@@ -1026,6 +1031,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       }
     }
     trace_mark(ctx, "symbolic");
+    LAMB_TRY(check_norm_index(mixed || filt_r));
     if (mixed) LAMB_TRY(build_work(ctx, C, sym, A, &work, &work_c, true));
     if (mixed || filt_r) LAMB_TRY(dalloc(ctx, &c_nrm, std::max<int64_t>(sym.c_nnz, 1)));
     trace_mark(ctx, "work items");

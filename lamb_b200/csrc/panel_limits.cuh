@@ -14,4 +14,8 @@ inline bool panel_blocks_ok(int64_t a_blocks, int64_t b_blocks, int64_t c_blocks
   return a_blocks <= kPanelMaxBlocks && b_blocks <= kPanelMaxBlocks && c_blocks <= kPanelMaxBlocks;
 }
 
+// The stack and the mixed kernels write block norms through a 32-bit index:
+// without norms (no result filter, FP64) a C may have more blocks.
+inline bool norm_index_ok(int64_t c_blocks, bool norms) { return !norms || c_blocks <= INT32_MAX; }
+
 }  // namespace lamb

@@ -18,6 +18,7 @@ int main(int argc, char** argv) {
   for (int i = 2; i < argc; ++i) v[i - 2] = atoll(argv[i]);
   bool ok = false;
   if (!strcmp(argv[1], "blocks")) ok = lamb::panel_blocks_ok(v[0], v[1], v[2]);
+  if (!strcmp(argv[1], "norms")) ok = lamb::norm_index_ok(v[0], v[1]);
   printf("%d\n", ok);
   return 0;
 }
@@ -44,3 +45,9 @@ def test_block_counts_fit_the_kernel_s_32_bits(rule):
         assert not rule("blocks", *v)
     # 51,200 atoms of one row, 5 % structured fill in A and B: C has every block
     assert not rule("blocks", 131072000, 131072000, 51200 * 51200)
+
+
+def test_block_norms_have_32_bit_indices(rule):
+    top = 2 ** 31 - 1
+    assert rule("norms", top, 1) and rule("norms", top + 1, 0)
+    assert not rule("norms", top + 1, 1)
