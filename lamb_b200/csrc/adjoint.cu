@@ -245,19 +245,22 @@ int32_t adjoint_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* dC, DevMat
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_WRONG_ARGS, "adjoint: outputs must be distinct matrices");
   // Group tiles where they win, as for the multiply: 384 waters (cutoff 6, both
   // products) 4.4 -> 2.8 ms a call, the stack building (1.2 ms) included.
-  bool panel = panel_worth(A, B) && dC->nnz > 0 && panel_blocks_ok(A->nnz, B->nnz, dC->nnz);
+  const bool worth = panel_worth(A, B) && dC->nnz > 0 && panel_blocks_ok(A->nnz, B->nnz, dC->nnz);
+  bool panel_a = worth && dA && panel_shapes_ok(A->h_row_bs, B->h_col_bs, A->h_col_bs);
+  bool panel_b = worth && dB && panel_shapes_ok(A->h_col_bs, A->h_row_bs, B->h_col_bs);
   std::shared_ptr<GroupTab> cols;
-  if (panel) {
+  if (panel_a || panel_b) {
     if (!A->h_pos.empty()) LAMB_TRY(ensure_row_order(ctx, A));  // the pattern's own order costs more than it gives here
     LAMB_TRY(product_groups(ctx, A, B, &cols));
-    panel = panel_gain(nullptr, *A->rgrp, *A->cgrp, *cols, A->h_row_bs, B->h_col_bs, 0, nullptr) >= kPanelGain;
+    if (panel_gain(nullptr, *A->rgrp, *A->cgrp, *cols, A->h_row_bs, B->h_col_bs, 0, nullptr) < kPanelGain)
+      panel_a = panel_b = false;
   }
   bool ran_a = false, ran_b = false;
   int64_t* odd = ctx->pin + kPinOdd;
   odd[0] = odd[1] = 0;
-  if (panel && dA)  // dA = dC . B^T: dC and B by rows, over the column atoms
+  if (panel_a)  // dA = dC . B^T: dC and B by rows, over the column atoms
     LAMB_TRY(masked_panels(ctx, A, dA, dC, true, B, true, A->rgrp, cols, A->cgrp, &odd[0], &ran_a));
-  if (panel && dB)  // dB = A^T . dC: A and dC by columns, over the row atoms
+  if (panel_b)  // dB = A^T . dC: A and dC by columns, over the row atoms
     LAMB_TRY(masked_panels(ctx, B, dB, A, false, dC, false, A->cgrp, A->rgrp, cols, &odd[1], &ran_b));
   if (ran_a || ran_b) {
     LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -1014,7 +1014,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       LAMB_TRY(pack_plane_meta(ctx, A, mp, &a_offk));
       LAMB_TRY(symbolic_phase(ctx, A, B, C, eps, filt_p, false, a_offk, &sym, mp.b_soff));
     } else {
-      if (panel_worth(A, B)) {
+      if (panel_worth(A, B) && panel_shapes_ok(A->h_row_bs, A->h_col_bs, B->h_col_bs)) {
         LAMB_TRY(product_groups(ctx, A, B, &c_grp));
         trace_mark(ctx, "atom groups");
         // queued before the count kernel: the totals arrive with the counts

@@ -960,18 +960,15 @@ double panel_gain(const PanelPair* p, const GroupTab& rows, const GroupTab& inne
   return per_pair * mean_slabs(row_bs) * mean_slabs(col_bs);
 }
 
-static bool panel_shapes_ok(const std::vector<int8_t>& rows, const std::vector<int8_t>& inner,
-                            const std::vector<int8_t>& cols) {
-  // 51,200 columns of single-atom groups are what the masks of one super row hold in shared memory
-  return !rows.empty() && !cols.empty() && !inner.empty() && max_block(rows) <= kGrpRows &&
-         max_block(inner) <= kGrpRows && max_block(cols) <= kGrpRows && cols.size() <= 51200 && rows.size() <= 262144 &&
-         inner.size() <= 65536;
+bool panel_shapes_ok(const std::vector<int8_t>& rows, const std::vector<int8_t>& inner,
+                     const std::vector<int8_t>& cols) {
+  return panel_atoms_ok((int64_t)rows.size(), (int64_t)inner.size(), (int64_t)cols.size()) &&
+         max_block(rows) <= kGrpRows && max_block(inner) <= kGrpRows && max_block(cols) <= kGrpRows;
 }
 
 bool panel_worth(const DevMatrix* A, const DevMatrix* B) {
   return A->n_cols > 0 && panel_blocks_ok(A->nnz, B->nnz, 0) &&
-         (double)A->nnz * B->nnz >= (double)(1 << 19) * A->n_cols &&
-         panel_shapes_ok(A->h_row_bs, A->h_col_bs, B->h_col_bs);
+         (double)A->nnz * B->nnz >= (double)(1 << 19) * A->n_cols;
 }
 
 int32_t product_groups(Ctx* ctx, DevMatrix* A, DevMatrix* B, std::shared_ptr<GroupTab>* cols) {

@@ -65,12 +65,17 @@ struct PanelPair {
   ~PanelPair();
 };
 
-// Whether the panel kernel may be considered for A.B (or its adjoint): its block
-// sizes, and about half a million block products (below that the launches that
-// prepare the panels, some 60 us, cost more than the stacks: 48 atoms of 0 to 3
-// rows, 53,000 products, 625 us a call with stacks, 690 us with panels; 64
-// waters, 1.6 million, even).
+// Whether the panel kernel may be considered for A.B (or its adjoint): about
+// half a million block products (below that the launches that prepare the
+// panels, some 60 us, cost more than the stacks: 48 atoms of 0 to 3 rows, 53,000
+// products, 625 us a call with stacks, 690 us with panels; 64 waters, 1.6
+// million, even).
 bool panel_worth(const DevMatrix* A, const DevMatrix* B);
+// Whether its tiles can hold the product of these row, inner and column atoms:
+// the roles of each product by itself (those of dA are A's rows, B's columns and
+// A's columns, those of dB A's columns, A's rows and B's columns).
+bool panel_shapes_ok(const std::vector<int8_t>& rows, const std::vector<int8_t>& inner,
+                     const std::vector<int8_t>& cols);
 // Groups of A.B's columns (those of its rows and inner atoms are A's): A's when
 // B lives on the same atoms (both then describe the same runs), B's own otherwise.
 int32_t product_groups(Ctx* ctx, DevMatrix* A, DevMatrix* B, std::shared_ptr<GroupTab>* cols);
