@@ -249,19 +249,29 @@ int32_t adjoint_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* dC, DevMat
   bool panel_a = worth && dA && panel_shapes_ok(A->h_row_bs, B->h_col_bs, A->h_col_bs);
   bool panel_b = worth && dB && panel_shapes_ok(A->h_col_bs, A->h_row_bs, B->h_col_bs);
   std::shared_ptr<GroupTab> cols;
+  // Panels that cannot be allocated leave the product to the stacks, with the
+  // scratch of this and earlier calls given back.
+  auto optional = [&](int32_t rc, bool* ran) -> int32_t {
+    if (!out_of_memory(rc)) return rc;
+    *ran = false;
+    release_scratch(ctx);
+    ctx->last_error.clear();
+    return LAMB_GPU_OK;
+  };
   if (panel_a || panel_b) {
     if (!A->h_pos.empty()) LAMB_TRY(ensure_row_order(ctx, A));  // the pattern's own order costs more than it gives here
-    LAMB_TRY(product_groups(ctx, A, B, &cols));
-    if (panel_gain(nullptr, *A->rgrp, *A->cgrp, *cols, A->h_row_bs, B->h_col_bs, 0, nullptr) < kPanelGain)
+    bool have = true;
+    LAMB_TRY(optional(product_groups(ctx, A, B, &cols), &have));
+    if (!have || panel_gain(nullptr, *A->rgrp, *A->cgrp, *cols, A->h_row_bs, B->h_col_bs, 0, nullptr) < kPanelGain)
       panel_a = panel_b = false;
   }
   bool ran_a = false, ran_b = false;
   int64_t* odd = ctx->pin + kPinOdd;
   odd[0] = odd[1] = 0;
   if (panel_a)  // dA = dC . B^T: dC and B by rows, over the column atoms
-    LAMB_TRY(masked_panels(ctx, A, dA, dC, true, B, true, A->rgrp, cols, A->cgrp, &odd[0], &ran_a));
+    LAMB_TRY(optional(masked_panels(ctx, A, dA, dC, true, B, true, A->rgrp, cols, A->cgrp, &odd[0], &ran_a), &ran_a));
   if (panel_b)  // dB = A^T . dC: A and dC by columns, over the row atoms
-    LAMB_TRY(masked_panels(ctx, B, dB, A, false, dC, false, A->cgrp, A->rgrp, cols, &odd[1], &ran_b));
+    LAMB_TRY(optional(masked_panels(ctx, B, dB, A, false, dC, false, A->cgrp, A->rgrp, cols, &odd[1], &ran_b), &ran_b));
   if (ran_a || ran_b) {
     LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     LAMB_TRY(check_tiles(ctx));

@@ -18,6 +18,7 @@ namespace lamb {
 
 // ---- status codes (level/type pairs of src/lamb_error.F90:120-159) -------
 inline int32_t make_status(int level, int type) { return level * 100000 + (type + 50000); }
+inline bool out_of_memory(int32_t status) { return status / 100000 == LAMB_LEVEL_MEMORY; }
 
 struct GroupTab;
 struct ClusterTab;

@@ -401,6 +401,17 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
   int64_t *s_cnt = c_cnt + n_rows, *p_cnt = s_cnt + n_rows;
   double* rfl = reinterpret_cast<double*>(p_cnt + n_rows);
   CountStat* d_stat = nullptr;
+  int64_t* s_row_base = nullptr;
+  struct Free {
+    Ctx* ctx;
+    int64_t **cnt, **base;
+    CountStat** stat;
+    ~Free() {
+      dfree(ctx, *cnt);
+      dfree(ctx, *base);
+      dfree(ctx, *stat);
+    }
+  } fr{ctx, &c_cnt, &s_row_base, &d_stat};
   LAMB_TRY(dalloc(ctx, &d_stat, 1));
   LAMB_CUDA(ctx, cudaMemsetAsync(d_stat, 0, sizeof(CountStat), ctx->stream));
   auto range = [](const DevMatrix* m) { return reinterpret_cast<const NormRange*>(m->norms + m->nnz); };
@@ -409,7 +420,7 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
   const size_t smem_count = sizeof(uint32_t) * (size_t)std::max(n_words, 1);
   if (smem_count > 200 * 1024)
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "too many block columns for the symbolic bitmap");
-  const bool keep_bits = (out->pattern_only || out->chunked_fill) && n_rows > 0 &&
+  const bool keep_bits = (out->pattern_only || out->chunked_fill) && !out->lean && n_rows > 0 &&
                          4 * (int64_t)n_rows * n_words <= kPatternBitsMax;
   if (keep_bits) LAMB_TRY(dalloc(ctx, &out->c_bm, (int64_t)n_rows * std::max(n_words, 1)));
   if (n_rows > 0) {
@@ -435,12 +446,7 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     LAMB_CUDA(ctx, cudaMemcpyAsync(ctx->pin + kPinCount, d_stat, sizeof(CountStat), cudaMemcpyDeviceToHost, ctx->stream));
     LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     // an operand may be the result of an asynchronous product that stopped
-    const int32_t rc = check_tiles(ctx);
-    if (rc != LAMB_GPU_OK) {
-      dfree(ctx, c_cnt);
-      dfree(ctx, d_stat);
-      return rc;
-    }
+    LAMB_TRY(check_tiles(ctx));
   }
   if (n_rows) {
     const CountStat& h = *reinterpret_cast<const CountStat*>(ctx->pin + kPinCount);
@@ -468,7 +474,6 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
   if (out->n_ent >= (1ll << 40) || max_s >= (1ll << 24))
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "stack too large");
   C->nnz = out->c_nnz;
-  int64_t* s_row_base = nullptr;
   LAMB_CUDA(ctx, cudaMemcpyAsync(C->row_p, h_crp, sizeof(int64_t) * (n_rows + 1), cudaMemcpyHostToDevice, ctx->stream));
   LAMB_TRY(dalloc(ctx, &C->col, std::max<int64_t>(C->nnz, 1)));
   if (!pattern_now) {
@@ -545,8 +550,6 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     LAMB_TRY(dalloc(ctx, &C->data, need));
     C->data_cap = need;
   }
-  dfree(ctx, c_cnt); dfree(ctx, s_row_base);
-  dfree(ctx, d_stat);
   trace_mark(ctx, "C data allocation");
   return LAMB_GPU_OK;
 }
@@ -906,7 +909,7 @@ static int32_t numeric_chunks(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C
 
 // ---- FP64 numeric phase on group tiles -------------------------------------------------
 // The tile kernel, in kMinChunks launches when a download may overlap them.
-// *ran = false (nothing done) when the panels do not fit.
+// *ran = false (nothing done) when the panels are too large.
 static int32_t numeric_panel(Ctx* ctx, DevMatrix* A, DevMatrix* C, const Symbolic& sym, PanelPair* pair, double eps,
                              double* c_nrm, bool overlap, bool* ran) {
   C->n_chunks = 0;
@@ -964,13 +967,16 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
   // LAMB_GPU_MIXED_MMA_SYNC=1 selects the mma.sync digit kernel for every shape.
   const char* force_sync = std::getenv("LAMB_GPU_MIXED_MMA_SYNC");
   bool tc_path = mixed && mixed_tc_eligible(A, B) && !(force_sync && force_sync[0] == '1');
-  sym.use_scratch = true;
   LAMB_TRY(settle(ctx));
   auto check_norm_index = [&](bool norms) -> int32_t {
     if (norm_index_ok(sym.c_nnz, norms)) return LAMB_GPU_OK;
     return fail(ctx, LAMB_LEVEL_FAILURE, LAMB_TYPE_UNIMPLEMENTED, "more than 2^31 blocks in a C with block norms");
   };
-  auto body = [&]() -> int32_t {
+  // lean: without the memory that another way does without (panels, their
+  // tables, bitmaps of C's pattern).
+  auto body = [&](bool lean) -> int32_t {
+    sym.use_scratch = true;
+    sym.lean = lean;
     trace_mark(ctx, "multiply: start");
     LAMB_TRY(check_compatible(ctx, A, B));
     LAMB_TRY(ensure_row_order(ctx, A));
@@ -1004,6 +1010,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       free_symbolic(ctx, sym);
       sym = Symbolic{};
       sym.use_scratch = true;
+      sym.lean = lean;
       if (timed) LAMB_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
     }
     if (mixed) {
@@ -1014,7 +1021,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
       LAMB_TRY(pack_plane_meta(ctx, A, mp, &a_offk));
       LAMB_TRY(symbolic_phase(ctx, A, B, C, eps, filt_p, false, a_offk, &sym, mp.b_soff));
     } else {
-      if (panel_worth(A, B) && panel_shapes_ok(A->h_row_bs, A->h_col_bs, B->h_col_bs)) {
+      if (!lean && panel_worth(A, B) && panel_shapes_ok(A->h_row_bs, A->h_col_bs, B->h_col_bs)) {
         LAMB_TRY(product_groups(ctx, A, B, &c_grp));
         trace_mark(ctx, "atom groups");
         // queued before the count kernel: the totals arrive with the counts
@@ -1056,11 +1063,27 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
     if (timed) LAMB_CUDA(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
     return LAMB_GPU_OK;
   };
-  int32_t rc = body();
-  free_slices(ctx, &mp);
-  dfree(ctx, a_offk);
-  dfree(ctx, c_nrm);
-  free_symbolic(ctx, sym);
+  auto drop = [&]() {
+    free_slices(ctx, &mp);
+    dfree(ctx, a_offk);
+    dfree(ctx, c_nrm);
+    free_symbolic(ctx, sym);
+    pair.release();
+  };
+  int32_t rc = body(false);
+  if (out_of_memory(rc)) {
+    // Once more on what the stacks need, with the scratch of earlier calls given back.
+    drop();
+    release_scratch(ctx);
+    mp = MixedPlanes{};
+    sym = Symbolic{};
+    c_grp.reset();
+    panel = false;
+    ctx->kern_chunks = 0;
+    ctx->last_error.clear();
+    rc = body(true);
+  }
+  drop();
   if (rc != LAMB_GPU_OK) return rc;
   C->norms_valid = false;
   // Without LAMB_GPU_ASYNC the filter's counts are applied now; with it the

@@ -41,6 +41,7 @@ struct Symbolic {
   std::vector<int64_t> h_base;     // C data offset of every (row subset, column subset, rank) run
   bool use_scratch = false;    // set before symbolic_phase: ent lives in the context's scratch
   bool pattern_only = false;   // set before symbolic_phase: C's pattern and layout only, no stacks
+  bool lean = false;           // set before symbolic_phase: keep no bitmaps (memory that another way does without)
   // set before symbolic_phase: C's pattern and layout now, the stacks later
   // one row chunk at a time (numeric_chunks); the fill's parameters are kept
   bool chunked_fill = false;

@@ -982,10 +982,11 @@ int32_t product_groups(Ctx* ctx, DevMatrix* A, DevMatrix* B, std::shared_ptr<Gro
   return LAMB_GPU_OK;
 }
 
-PanelPair::~PanelPair() {
+void PanelPair::release() {
   for (PanelSide* s : {&a, &b}) {
     if (s->buf) cudaFreeAsync(s->buf, ctx->stream);
     if (s->buf2) cudaFreeAsync(s->buf2, ctx->stream);
+    s->buf = s->buf2 = nullptr;
   }
 }
 
@@ -1073,7 +1074,7 @@ int32_t panel_pack(Ctx* ctx, PanelPair* p, const int64_t* totals, bool filt, boo
     s.kc = reinterpret_cast<int32_t*>(d);
     s.sbg = s.kc + n;
     s.mask = reinterpret_cast<uint32_t*>(s.sbg + n);
-    if (scratch(ctx, slot[k], n * p->kstride * kW, &s.panel) != LAMB_GPU_OK) return LAMB_GPU_OK;
+    LAMB_TRY(scratch(ctx, slot[k], n * p->kstride * kW, &s.panel));
   }
   PairArgs r = pair_args(*p);
   const int outs = std::max(p->a.out->n, p->b.out->n), sbs = std::max(p->a.n_sb, p->b.n_sb);

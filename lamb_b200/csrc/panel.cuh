@@ -62,7 +62,8 @@ struct PanelPair {
   // device: superblocks of a and b, superblock pairs, and (after the packing)
   // whether a value is infinite or NaN
   int64_t* totals = nullptr;
-  ~PanelPair();
+  void release();  // gives the device buffers back (stream-ordered)
+  ~PanelPair() { release(); }
 };
 
 // Whether the panel kernel may be considered for A.B (or its adjoint): about
@@ -96,7 +97,9 @@ int32_t panel_index(Ctx* ctx, PanelPair* p, const DevMatrix* ma, bool a_rows_out
                     std::shared_ptr<GroupTab> out_a, std::shared_ptr<GroupTab> in, std::shared_ptr<GroupTab> out_b,
                     int64_t* totals);
 // Panels of both operands (after the totals have arrived); filt: with block
-// norms.  *ok = false, and nothing queued, when they are too large.
+// norms.  *ok = false, and nothing queued, when they are too large.  What cannot
+// be allocated, here or in the other calls, is the callers' to do without: they
+// give the memory back and take the stacks.
 int32_t panel_pack(Ctx* ctx, PanelPair* p, const int64_t* totals, bool filt, bool* ok);
 // Pattern bitmap of Z for panel_tiles (freed by the caller).
 int32_t panel_pattern(Ctx* ctx, const DevMatrix* Z, uint32_t** bm, int32_t** pre);
