@@ -216,6 +216,7 @@ static int32_t masked_panels(Ctx* ctx, const DevMatrix* Z, DevMatrix* out, const
                              const DevMatrix* m2, bool rows2, std::shared_ptr<GroupTab> out1,
                              std::shared_ptr<GroupTab> in, std::shared_ptr<GroupTab> out2, int64_t* odd, bool* ran) {
   *ran = false;
+  ScratchUse use(ctx);
   PanelPair pair;
   LAMB_TRY(panel_index(ctx, &pair, m1, rows1, m2, rows2, out1, in, out2, ctx->pin + kPinPanel));
   LAMB_TRY(masked_output(ctx, Z, out));

@@ -121,8 +121,10 @@ struct Ctx {
   // Multiply temporaries of several GB (stacks, work items, digit planes) are
   // kept between calls: releasing and re-reserving them fragments the
   // stream-ordered pool, which then maps fresh memory at up to a second a call.
+  // They go back when an allocation of the context fails while no call uses them.
   void* scr[kScrSlots] = {};
   size_t scr_bytes[kScrSlots] = {};
+  int scr_users = 0;  // ScratchUse objects alive
   // Result filter whose host metadata is still on its way (LAMB_GPU_ASYNC):
   // per-sector kept block counts land in pend_h (pinned) when pend_ev fires.
   DevMatrix* pend_m = nullptr;
@@ -188,8 +190,8 @@ int32_t fail(Ctx* ctx, int level, int type, const std::string& msg);
   } while (0)
 
 // Stream-ordered allocation on the context's stream.  When the pool cannot
-// satisfy a request, unused pool memory is returned to the device once and the
-// allocation retried.
+// satisfy a request, idle scratch and unused pool memory are returned to the
+// device once and the allocation retried.
 int32_t dalloc_bytes(Ctx* ctx, void** p, size_t bytes);
 template <typename T>
 int32_t dalloc(Ctx* ctx, T** p, int64_t n) {
@@ -206,6 +208,15 @@ int32_t scratch(Ctx* ctx, int slot, int64_t n, T** p) {
   return scratch_bytes(ctx, slot, sizeof(T) * (size_t)std::max<int64_t>(n, 1), reinterpret_cast<void**>(p));
 }
 void release_scratch(Ctx* ctx);
+// Alive while scratch buffers are in use: from before the first is asked for
+// until the last launch that uses one is queued.
+struct ScratchUse {
+  Ctx* ctx;
+  explicit ScratchUse(Ctx* c) : ctx(c) { ++ctx->scr_users; }
+  ~ScratchUse() { --ctx->scr_users; }
+  ScratchUse(const ScratchUse&) = delete;
+  ScratchUse& operator=(const ScratchUse&) = delete;
+};
 // Grow-only pinned buffer of the context for one role.
 int32_t pinned_bytes(Ctx* ctx, int slot, size_t bytes, void** p);
 template <typename T>

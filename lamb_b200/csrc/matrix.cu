@@ -30,6 +30,7 @@ int32_t dalloc_bytes(Ctx* ctx, void** p, size_t bytes) {
   cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
+    if (ctx->scr_users == 0) release_scratch(ctx);
     cudaMemPool_t pool;
     if (cudaStreamSynchronize(ctx->stream) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess &&
         cudaMemPoolTrimTo(pool, 0) == cudaSuccess)

@@ -975,6 +975,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
   // lean: without the memory that another way does without (panels, their
   // tables, bitmaps of C's pattern).
   auto body = [&](bool lean) -> int32_t {
+    ScratchUse use(ctx);
     sym.use_scratch = true;
     sym.lean = lean;
     trace_mark(ctx, "multiply: start");

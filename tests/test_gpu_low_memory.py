@@ -36,6 +36,14 @@ def test_stacks_where_panels_do_not_fit(shim, case):
     _run(shim, case)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["upload", "copy", "adjoint_stacks"])
+def test_idle_scratch_is_given_back(shim, how):
+    """The panels of a finished product stay with the context, but not when
+    something else needs the memory."""
+    _run(shim, "idle_" + how)
+
+
 # ---- the child process ------------------------------------------------------------------
 def _band(rng, n, sizes, width):
     """Atoms in runs of len(sizes) that couple to the same atoms, `width` runs to either side."""
@@ -59,12 +67,52 @@ def _bytes_of(sizes):
     return sum(8 * (s.n_rows + 1) + 12 * s.n_blks + 8 * s.data_len for s in sizes)
 
 
+def _idle(gpu, mem, case):
+    rng = np.random.default_rng(1)
+    a, b = _band(rng, 1300, [13, 5, 5], 10), _band(rng, 1300, [13, 5, 5], 10)
+    ctx = gpu.Context(0)
+    da, db = ctx.upload(a), ctx.upload(b)
+    dc = ctx.create_like(da)
+    ctx.synchronize()
+    held = mem.low_memory_live()
+    ctx.multiply(da, db, dc, 0.0)
+    c_bytes = _bytes_of(dc.sizes())
+    kept = mem.low_memory_live() - held - c_bytes
+    assert kept > 200 * MB  # the panels
+    want = dc.download()
+    # room for less than a second C beside the panels, and for more than one without them
+    mem.low_memory_limit(held + c_bytes + kept + c_bytes // 2)
+    if case == "idle_upload":
+        m = ctx.upload(want)
+    elif case == "idle_copy":
+        m = ctx.create_like(dc)
+        ctx.copy(dc, m)
+    else:  # blocks of 25 rows take no panels: results of 2 x 100 MB, stacks of 40 MB
+        mem.low_memory_limit(1 << 62)
+        x = [ctx.upload(_band(rng, 700, [25, 5], 10)) for _ in range(3)]
+        ga, gb = ctx.create_like(x[0]), ctx.create_like(x[1])
+        mem.low_memory_limit(mem.low_memory_live() + 100 * MB)
+        ctx.adjoint(*x, ga, gb)
+        m = dc
+    got = m.download()
+    for s, t in zip(got.sectors, want.sectors):
+        assert np.array_equal(s.data, t.data) and np.array_equal(s.col_i, t.col_i)
+    # and the next product makes its panels again
+    mem.low_memory_limit(ctypes.c_size_t(-1).value)
+    ctx.multiply(da, db, dc, 0.0)
+    for s, t in zip(dc.download().sectors, want.sectors):
+        assert np.array_equal(s.data, t.data)
+    ctx.close()
+
+
 def _child(path, case):
     from lamb_b200 import gpu
     mem = ctypes.CDLL(path)
     for f in ("low_memory_live", "low_memory_peak"):
         getattr(mem, f).restype = ctypes.c_size_t
     mem.low_memory_limit.argtypes = [ctypes.c_size_t]
+    if case.startswith("idle"):
+        return _idle(gpu, mem, case)
     none = ctypes.c_size_t(-1).value
     rng = np.random.default_rng(1)
     # `stacks`: what the stack kernel's entries, work items and tables take, generously
