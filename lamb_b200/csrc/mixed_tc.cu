@@ -1257,7 +1257,7 @@ static int32_t make_clusters(Ctx* ctx, const int32_t* order, const std::vector<i
     const int64_t I = t->n - 1;
     of[a] = (int32_t)I;
     idx[a] = atoms;
-    off[a] = rows;
+    off[a] = b > 0 ? rows : 0;  // an atom without elements may follow the last row: 128 has no place in 7 bits
     if (cols) cab[I * kMaxColAtoms + atoms] = rows | (b << 8);
     for (int e = 0; e < b; ++e) {
       geo[I * max_rows + rows + e] = (atoms << 16) | (e << 8) | b;
