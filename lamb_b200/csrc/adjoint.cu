@@ -279,13 +279,17 @@ int32_t adjoint_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* dC, DevMat
     ran_a = ran_a && !odd[0];
     ran_b = ran_b && !odd[1];
   }
+  if (dA && ran_a) trace_mark(ctx, "dA (group tiles)");
+  if (dB && ran_b) trace_mark(ctx, "dB (group tiles)");
   if (dA && !ran_a) {
+    trace_mark(ctx, "dA (stacks)");
     LAMB_TRY(masked_output(ctx, A, dA));
     // dA_ik = sum_j dC_ij . B_kj^T: rows of dC and rows of B, op2 transposed.
     LAMB_TRY(masked_product(ctx, dA, dC->row_p, dC->col, nullptr, dC->off, dC->data, B->row_p, B->col, nullptr,
                             B->off, B->data, dC->col_bs, max_block(dC->h_col_bs), false, true));
   }
   if (dB && !ran_b) {
+    trace_mark(ctx, "dB (stacks)");
     LAMB_TRY(masked_output(ctx, B, dB));
     // dB_kj = sum_i A_ik^T . dC_ij: columns of A and of dC, op1 transposed.
     TIndex at, ct;

@@ -1057,7 +1057,7 @@ int32_t multiply_impl(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, double
         LAMB_TRY(numeric_chunks(ctx, A, B, C, sym, a_offk, c_nrm));
       }
     }
-    trace_mark(ctx, "numeric");
+    trace_mark(ctx, mixed ? "numeric (mma.sync digits)" : panel ? "numeric (group tiles)" : "numeric (stacks)");
     if (timed) LAMB_CUDA(ctx, cudaEventRecord(ctx->ev[2], ctx->stream));
     if (filt_r) LAMB_TRY(result_filter(ctx, C, c_nrm, eps));
     trace_mark(ctx, "result filter");
