@@ -340,6 +340,15 @@ struct Walk {
 __device__ __forceinline__ int64_t global_warp() { return ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
 __device__ __forceinline__ int64_t grid_warps() { return ((int64_t)gridDim.x * blockDim.x) >> 5; }
 
+// Lets a kernel take `bytes` of dynamic shared memory.  The 48 KB that need no
+// asking include its static shared memory (a few KB), so it asks early.
+template <typename K>
+int32_t allow_smem(Ctx* ctx, K kern, size_t bytes) {
+  if (bytes > 32 * 1024)
+    LAMB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return LAMB_GPU_OK;
+}
+
 constexpr int kThreads = 256;
 // Counts a launch of one of this library's kernels and checks it.
 #define LAMB_LAUNCHED(ctx) do { ++(ctx)->launches; LAMB_CUDA((ctx), cudaGetLastError()); } while (0)

@@ -537,8 +537,7 @@ int32_t numeric_mixed(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, const 
   const int cap = std::max(1, std::min(32, 4096 / wpe));
   const int tbl_words = cap * wpe;
   const size_t smem = sizeof(WordRef) * (size_t)tbl_words * kMixWarps;
-  if (smem > 48 * 1024)
-    LAMB_CUDA(ctx, cudaFuncSetAttribute(k_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LAMB_TRY(allow_smem(ctx, k_mixed, smem));
   int sms = 148, per_sm = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   LAMB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mixed, kMixWarps * 32, smem));

@@ -426,8 +426,7 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
   if (n_rows > 0) {
     const bool few = n_rows < kSymFewRows;
     auto count_kern = few ? k_sym_count<1024> : k_sym_count<kSymThreads>;
-    if (smem_count > 48 * 1024)
-      LAMB_CUDA(ctx, cudaFuncSetAttribute(count_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
+    LAMB_TRY(allow_smem(ctx, count_kern, smem_count));
     int grid = 1;
     LAMB_TRY(resident_grid(ctx, count_kern, smem_count, n_rows, &grid, few ? 1024 : kSymThreads));
     count_kern<<<grid, few ? 1024 : kSymThreads, smem_count, ctx->stream>>>(
@@ -510,8 +509,7 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
     if (!out->want_bits) dfree(ctx, out->c_bm);
   } else if (pattern_now && n_rows > 0 && C->nnz > 0) {
     const size_t smem_pat = sizeof(uint32_t) * 2 * (size_t)std::max(n_words, 1);
-    if (smem_pat > 48 * 1024)
-      LAMB_CUDA(ctx, cudaFuncSetAttribute(k_sym_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_pat));
+    LAMB_TRY(allow_smem(ctx, k_sym_pattern, smem_pat));
     int pgrid = 1;
     LAMB_TRY(resident_grid(ctx, k_sym_pattern, smem_pat, n_rows, &pgrid));
     k_sym_pattern<<<pgrid, kSymThreads, smem_pat, ctx->stream>>>(n_rows, A->row_p, A->col, A->norms, B->row_p, B->col,
@@ -522,8 +520,7 @@ int32_t symbolic_phase(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, doubl
   }
   if (!pattern_now && n_rows > 0 && C->nnz > 0) {
     auto kern = want_ids ? k_sym_fill<true> : k_sym_fill<false>;
-    if (smem_fill > 48 * 1024)
-      LAMB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fill));
+    LAMB_TRY(allow_smem(ctx, kern, smem_fill));
     // As many CTAs as fit at once (6 per SM at 40 registers): CTAs of a larger
     // grid start only when a resident one has finished all its rows (a grid
     // of 8 per SM took 1.8 ms longer at 6,144 waters).
@@ -795,8 +792,7 @@ static int32_t numeric_chunks(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C
   // the fill keeps resident, so that it fills the GPU (few heavy rows, as in
   // the products of dense density matrices, would otherwise leave most SMs idle).
   auto fill = k_sym_fill<false>;
-  if (sym.fill_smem > 48 * 1024)
-    LAMB_CUDA(ctx, cudaFuncSetAttribute(fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sym.fill_smem));
+  LAMB_TRY(allow_smem(ctx, fill, sym.fill_smem));
   int fgrid_all = 1;
   LAMB_TRY(resident_grid(ctx, fill, sym.fill_smem, n, &fgrid_all));
   const int min_rows = std::max(1, fgrid_all);

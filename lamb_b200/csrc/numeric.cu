@@ -350,8 +350,7 @@ static int32_t launch_batch_nw(Ctx* ctx, int64_t n_work, const Work* work, const
   const int tbl_cols = cap * mi;
   const size_t smem = sizeof(ColRef) * (size_t)tbl_cols * NW;
   auto kern = k_stacked_batch<NW>;
-  if (smem > 48 * 1024)
-    LAMB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LAMB_TRY(allow_smem(ctx, kern, smem));
   int sms = 148, per_sm = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   LAMB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NW * 32, smem));
@@ -377,8 +376,7 @@ static int32_t launch_stacked(Ctx* ctx, int64_t n_work, const Work* work, const 
   const int tbl_cols = cap * mi;
   const size_t smem = sizeof(ColRef) * (size_t)tbl_cols * kNumWarps;
   auto kern = k_stacked<TA, TB>;
-  if (smem > 48 * 1024)
-    LAMB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LAMB_TRY(allow_smem(ctx, kern, smem));
   int sms = 148, per_sm = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   LAMB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kNumWarps * 32, smem));

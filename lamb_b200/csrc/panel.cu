@@ -1152,8 +1152,7 @@ int32_t panel_tiles(Ctx* ctx, const PanelPair& p, const DevMatrix* C, const uint
   q.count = reinterpret_cast<int32_t*>(q.items + n_items);
   LAMB_CUDA(ctx, cudaMemsetAsync(q.count + n_sup + 1, 0, sizeof(int32_t) * kMaxChunks, ctx->stream));
   const size_t msk = 8 * (size_t)n_mj;
-  if (msk > 48 * 1024)
-    LAMB_CUDA(ctx, cudaFuncSetAttribute(k_panel_masks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msk));
+  LAMB_TRY(allow_smem(ctx, k_panel_masks, msk));
   k_panel_masks<<<n_sup, 512, msk, ctx->stream>>>(q);
   LAMB_LAUNCHED(ctx);
   k_panel_mask_scan<<<1, 1024, 0, ctx->stream>>>(n_sup, q.count);
