@@ -151,7 +151,7 @@ constexpr int kPinCount = 0;    // what the symbolic count leaves (CountStat, 5 
 constexpr int kPinPanel = 5;    // panel totals
 constexpr int kPinOdd = 8;       // non-finite values met while packing (the adjoint's two products)
 constexpr int kPinTileErr = 10;  // tile_err after the last panel product
-constexpr int kPinTc = 16;       // sizes, statistics and error code of the mixed tiles (9 words)
+constexpr int kPinTc = 16;       // sizes, statistics and error code of the mixed tiles (10 words)
 constexpr int kPinWords = 64;
 // The smallest and the largest of a matrix's block norms, as bit patterns that
 // an atomic maximum can collect (norms are >= 0 or NaN; a NaN is the largest).
