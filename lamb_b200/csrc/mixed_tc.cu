@@ -336,43 +336,44 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tc_tiles(TcArgs g) {
     // chunk v % 4): consecutive lanes copy consecutive chunks of one panel
     // row, so a warp reads whole 128-byte (A) or 64-byte (B) rows.
     // A lane whose wait ran out copies nothing more and leaves with its warp at
-    // the vote that every stage has anyway (the rows are read before lane 0
-    // gives them back): a vote at each wait cost 1 % of the mixed multiply.
-    bool go = true;
+    // the vote after the stage's copies, which also shows that every lane has
+    // read its rows: a vote at each wait cost 1 % of the mixed multiply.
     for (int64_t gs = 0;; ++gs) {
       const int ring = (int)(gs % kRing), stg = (int)(gs % kStages);
-      go = go && bar_wait<true>(&sm->bar_row_full[ring], (uint32_t)((gs / kRing) & 1), sm, g.err, kErrTimeoutRows);
+      bool go = bar_wait<true>(&sm->bar_row_full[ring], (uint32_t)((gs / kRing) & 1), sm, g.err, kErrTimeoutRows);
       int2 prow[kUnits / kProducers];
 #pragma unroll
       for (int i = 0; i < kUnits / kProducers; ++i) {
         const int u = pt + kProducers * i;
         prow[i] = sm->rows[ring][u < 256 ? (u >> 3) : ((u - 256) >> 2)];
       }
-      if (!__all_sync(0xffffffffu, go && prow[0].x != kEndRow)) break;
-      if (lane == 0) bar_arrive(&sm->bar_row_empty[ring]);
-      go = bar_wait<true>(&sm->bar_empty[stg], (uint32_t)(((gs / kStages) & 1) ^ 1), sm, g.err, kErrTimeoutEmpty);
-      if (!go) continue;
-      const uint32_t sa = smem_u32(stages + (size_t)stg * kStageBytes);
-      const uint32_t sb = sa + kStageA;
+      go = go && prow[0].x != kEndRow &&
+           bar_wait<true>(&sm->bar_empty[stg], (uint32_t)(((gs / kStages) & 1) ^ 1), sm, g.err, kErrTimeoutEmpty);
+      if (go) {
+        const uint32_t sa = smem_u32(stages + (size_t)stg * kStageBytes);
+        const uint32_t sb = sa + kStageA;
 #pragma unroll
-      for (int i = 0; i < kUnits / kProducers; ++i) {
-        const int u = pt + kProducers * i;
-        const bool is_a = u < 256;  // uniform over the warp
-        const int row = is_a ? (u >> 3) : ((u - 256) >> 2);
-        const int ch = is_a ? (u & 7) : ((u - 256) & 3);
-        const bool valid = prow[i].x >= 0;
-        const uint32_t bytes = valid ? 16u : 0u;
-        if (is_a) {
-          const int8_t* src = g.pan_a + (int64_t)(valid ? prow[i].x : 0) * 128 + 16 * ch;
+        for (int i = 0; i < kUnits / kProducers; ++i) {
+          const int u = pt + kProducers * i;
+          const bool is_a = u < 256;  // uniform over the warp
+          const int row = is_a ? (u >> 3) : ((u - 256) >> 2);
+          const int ch = is_a ? (u & 7) : ((u - 256) & 3);
+          const bool valid = prow[i].x >= 0;
+          const uint32_t bytes = valid ? 16u : 0u;
+          if (is_a) {
+            const int8_t* src = g.pan_a + (int64_t)(valid ? prow[i].x : 0) * 128 + 16 * ch;
 #pragma unroll
-          for (int p = 0; p < kS; ++p) cp16(sa + p * kPlaneA + a_swz(row, ch), src + p * g.plane_a, bytes);
-        } else {
-          const int8_t* src = g.pan_b + (int64_t)(valid ? prow[i].y : 0) * 64 + 16 * ch;
+            for (int p = 0; p < kS; ++p) cp16(sa + p * kPlaneA + a_swz(row, ch), src + p * g.plane_a, bytes);
+          } else {
+            const int8_t* src = g.pan_b + (int64_t)(valid ? prow[i].y : 0) * 64 + 16 * ch;
 #pragma unroll
-          for (int p = 0; p < kS; ++p) cp16(sb + p * kPlaneB + b_swz(row, ch), src + p * g.plane_b, bytes);
+            for (int p = 0; p < kS; ++p) cp16(sb + p * kPlaneB + b_swz(row, ch), src + p * g.plane_b, bytes);
+          }
         }
+        cp_arrive(&sm->bar_full[stg]);
       }
-      cp_arrive(&sm->bar_full[stg]);
+      if (!__all_sync(0xffffffffu, go)) break;
+      if (lane == 0) bar_arrive(&sm->bar_row_empty[ring]);
     }
     // copies that no stage waited for (after an abort) land before the CTA ends
     asm volatile("cp.async.wait_all;" ::: "memory");
