@@ -629,23 +629,28 @@ static void cuthill_mckee(int n, const std::vector<int64_t>& rp, const std::vect
   };
   std::vector<char> seen(n, 0);
   std::vector<int32_t> nb;
-  for (int start = 0; start < n; ++start)
-    while (!seen[start]) {  // in a one-directional pattern `start` need not be reached from the row found for it
-      int s = bfs_last(bfs_last(start));
-      if (seen[s]) s = start;
-      size_t h = order.size();
-      order.push_back(s);
-      seen[s] = 1;
-      for (; h < order.size(); ++h) {
-        nb.clear();
-        for (int64_t b = rp[order[h]]; b < rp[order[h] + 1]; ++b) {
-          int j = cl[b];
-          if (j < n && !seen[j]) { seen[j] = 1; nb.push_back(j); }
-        }
-        std::sort(nb.begin(), nb.end(), [&](int x, int y) { return deg[x] < deg[y] || (deg[x] == deg[y] && x < y); });
-        order.insert(order.end(), nb.begin(), nb.end());
+  auto add_from = [&](int s) {
+    size_t h = order.size();
+    order.push_back(s);
+    seen[s] = 1;
+    for (; h < order.size(); ++h) {
+      nb.clear();
+      for (int64_t b = rp[order[h]]; b < rp[order[h] + 1]; ++b) {
+        int j = cl[b];
+        if (j < n && !seen[j]) { seen[j] = 1; nb.push_back(j); }
       }
+      std::sort(nb.begin(), nb.end(), [&](int x, int y) { return deg[x] < deg[y] || (deg[x] == deg[y] && x < y); });
+      order.insert(order.end(), nb.begin(), nb.end());
     }
+  };
+  for (int start = 0; start < n; ++start) {
+    if (seen[start]) continue;
+    const int s = bfs_last(bfs_last(start));
+    add_from(seen[s] ? start : s);
+  }
+  // in a one-directional pattern `start` need not be reached from the row found for it
+  for (int start = 0; start < n; ++start)
+    if (!seen[start]) add_from(start);
 }
 
 int32_t ensure_row_order(Ctx* ctx, DevMatrix* m) {
