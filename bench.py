@@ -440,7 +440,8 @@ def run_ours(args):
                          "traffic_scope": "DRAM bytes of one multiply's tile-kernel launch, scaled by block products "
                                           "from the committed small-case capture; null when none",
                          "flops_per_multiply": flops, "ms_per_multiply": ms_kern,
-                         "timing": "CUDA events around the product kernel's launches, summed per multiply; "
+                         "timing": "CUDA events around the product kernel's launches (k_panel_tiles: the atoms of water "
+                                   "boxes form groups), summed per multiply; "
                                    "numeric phase with the panels' packing: "
                                    f"{ms_num:.2f} ms"},
             "roofline_hbm": {"bound": "hbm", "achieved": alg_bytes / (ms_tot * 1e-3) / 1e9,

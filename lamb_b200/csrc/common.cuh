@@ -267,7 +267,6 @@ void free_sector_index(Ctx* ctx, SectorIndex* si);
 // Exclusive scan of int64 (in place allowed), via CUB with stream-ordered scratch.
 int32_t exclusive_scan_i64(Ctx* ctx, const int64_t* in, int64_t* out, int64_t n);
 int32_t inclusive_scan_i64(Ctx* ctx, const int64_t* in, int64_t* out, int64_t n);
-int32_t sum_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out);
 // Largest of n int64 (waits for the stream); 0 when n == 0.
 int32_t max_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out);
 

@@ -271,24 +271,6 @@ int32_t inclusive_scan_i64(Ctx* ctx, const int64_t* in, int64_t* out, int64_t n)
   return LAMB_GPU_OK;
 }
 
-int32_t sum_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out) {
-  *host_out = 0;
-  if (n <= 0) return LAMB_GPU_OK;
-  int64_t* d_out = nullptr;
-  LAMB_TRY(dalloc(ctx, &d_out, 1));
-  size_t bytes = 0;
-  LAMB_CUDA(ctx, cub::DeviceReduce::Sum(nullptr, bytes, in, d_out, n, ctx->stream));
-  void* tmp = nullptr;
-  LAMB_TRY(dalloc(ctx, (char**)&tmp, (int64_t)bytes + 16));
-  cudaError_t e = cub::DeviceReduce::Sum(tmp, bytes, in, d_out, n, ctx->stream);
-  cudaFreeAsync(tmp, ctx->stream);
-  LAMB_CUDA(ctx, e);
-  LAMB_CUDA(ctx, cudaMemcpyAsync(host_out, d_out, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  dfree(ctx, d_out);
-  return LAMB_GPU_OK;
-}
-
 int32_t max_i64(Ctx* ctx, const int64_t* in, int64_t n, int64_t* host_out) {
   *host_out = 0;
   if (n <= 0) return LAMB_GPU_OK;

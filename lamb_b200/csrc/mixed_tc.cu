@@ -264,16 +264,6 @@ __device__ __forceinline__ void mma_commit(unsigned long long* b) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, int (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
-      "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -1107,7 +1097,7 @@ __global__ void k_tc_cluster_exp(int64_t n, const int32_t* __restrict__ elem, co
     out[x] = elem[x] >= 0 ? e[elem[x]] : 0;
 }
 
-// ---- host ----------------------------------------------------------------------------------
+// ---- clusters ------------------------------------------------------------------------------
 // Clusters of nearby atoms.  A tile's inner dimension is the union of what its
 // atoms couple to, so its work grows with the extent of its clusters; cutting
 // the processing order (a Morton curve) into runs leaves clusters that straddle
@@ -1218,7 +1208,6 @@ __global__ void __launch_bounds__(32) k_tc_pool(int32_t n, int32_t ranges, const
   }
 }
 
-// ---- host ----------------------------------------------------------------------------------
 }  // namespace tc
 
 // Clusters of one axis with the tables the kernels read, in one device buffer.
@@ -1240,8 +1229,8 @@ struct ClusterTab {
 
 namespace tc {
 
-// Cuts `order` into clusters of at most max_rows rows and max_atoms atoms, and
-// before every complemented atom of it.
+// Cuts `order` into clusters: a new one where the next atom would pass max_rows
+// rows or max_atoms atoms, and before every complemented atom.
 static int32_t make_clusters(Ctx* ctx, const int32_t* order, const std::vector<int8_t>& bs, bool cols,
                              std::shared_ptr<ClusterTab>* out) {
   const int max_rows = cols ? kN : kM, max_atoms = cols ? kMaxColAtoms : kMaxRowAtoms;
@@ -1367,7 +1356,7 @@ int32_t numeric_mixed_tc(Ctx* ctx, DevMatrix* A, DevMatrix* B, DevMatrix* C, con
   const ClusterTab &rc = *A->rclu, &cc = *ccp;
   const int32_t nk = A->n_cols, W = (nk + 31) / 32;
   Bufs m{ctx, {}};
-  const int32_t *d_rcl = rc.of, *d_ratom = rc.idx, *d_roff = rc.off, *d_ccl = cc.of, *d_catom = cc.idx, *d_coff = cc.off;
+  const int32_t *d_rcl = rc.of, *d_ratom = rc.idx, *d_roff = rc.off, *d_ccl = cc.of, *d_catom = cc.idx;
   int32_t *d_rc_exp, *d_cc_exp;
   LAMB_TRY(m.alloc(&d_rc_exp, (int64_t)rc.n * kM)); LAMB_TRY(m.alloc(&d_cc_exp, (int64_t)cc.n * kN));
   k_tc_cluster_exp<<<grid_for((int64_t)rc.n * kM), 256, 0, ctx->stream>>>((int64_t)rc.n * kM, rc.elem, mp.ea, d_rc_exp);

@@ -357,7 +357,7 @@ struct TileSide {
   const double2* nrange;
   const double* nrm;
   const double* panel;
-  const int32_t *order, *first, *rows, *arow;
+  const int32_t *first, *rows;
   const uint16_t* geo;  // GroupTab::geo
   int32_t max_atoms;
 };
@@ -837,7 +837,7 @@ std::vector<int32_t> cut_groups(const std::vector<int8_t>& bs, const std::vector
 
 // Device tables of the runs `first`; ranks by the smallest processing position
 // of a run's atoms (order empty: as they come).
-int32_t make_groups(Ctx* ctx, std::vector<int32_t> first, const std::vector<int8_t>& bs,
+int32_t make_groups(Ctx* ctx, const std::vector<int32_t>& first, const std::vector<int8_t>& bs,
                     const std::vector<int32_t>& order, std::shared_ptr<GroupTab>* out) {
   auto t = std::make_shared<GroupTab>();
   t->ctx = ctx;
@@ -879,7 +879,6 @@ int32_t make_groups(Ctx* ctx, std::vector<int32_t> first, const std::vector<int8
     hr[key[x].second] = x;
     t->h_minpos[x] = key[x].first;
   }
-  t->h_first = std::move(first);
   LAMB_TRY(dalloc(ctx, &t->first, (int64_t)h.size()));
   LAMB_CUDA(ctx, cudaMemcpyAsync(t->first, h.data(), sizeof(int32_t) * h.size(), cudaMemcpyHostToDevice, ctx->stream));
   LAMB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // h dies here
@@ -1164,8 +1163,8 @@ int32_t panel_tiles(Ctx* ctx, const PanelPair& p, const DevMatrix* C, const uint
   const PanelSide* sd[2] = {&p.a, &p.b};
   for (int k = 0; k < 2; ++k) {
     const PanelSide& x = *sd[k];
-    t.s[k] = TileSide{x.bm, x.pre, x.ptr, x.mask, x.nrange, x.nrm, x.panel, x.out->order, x.out->first, x.out->rows,
-                      x.out->arow, x.out->geo, x.out->max_atoms};
+    t.s[k] = TileSide{x.bm, x.pre, x.ptr, x.mask, x.nrange, x.nrm, x.panel, x.out->first, x.out->rows,
+                      x.out->geo, x.out->max_atoms};
   }
   t.words = p.b.words; t.kstride = p.kstride;
   t.c_words = (C->n_cols + 31) / 32; t.c_bm = c_bm; t.c_pre = c_pre;

@@ -15,7 +15,6 @@ struct GroupTab {
   int32_t n = 0, n_atoms = 0;
   int32_t max_rows = 0, max_atoms = 0;  // of any group
   bool ordered = false;                 // ranks follow a processing order (otherwise the atoms' own)
-  std::vector<int32_t> h_first;         // [n + 1] first atom of every group
   std::vector<int32_t> h_minpos;        // [n] by rank: smallest processing position of the group's atoms
   // one device buffer holding, in this order:
   int32_t* first = nullptr;  // [n + 1]
