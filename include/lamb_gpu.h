@@ -158,6 +158,7 @@ typedef int64_t lamb_gpu_matrix; /* handle, > 0 when valid */
  * device buffers that back lamb_data_X/lamb_index storage on the GPU
  * (ownership mirrors lamb_data_X_type%mine, src/lamb_data_X_types.F90:80). */
 LAMB_API int32_t lamb_gpu_ctx_create(int32_t device, lamb_gpu_ctx** ctx);
+/* Also reports an asynchronous product that stopped and that no call reported. */
 LAMB_API int32_t lamb_gpu_ctx_destroy(lamb_gpu_ctx* ctx);
 /* Copies the last error message (NUL-terminated, truncated to len). */
 LAMB_API int32_t lamb_gpu_last_error(const lamb_gpu_ctx* ctx, char* msg, int32_t len);

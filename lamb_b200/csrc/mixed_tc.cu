@@ -37,7 +37,8 @@
 //   warps 0-5  producers: gather the tile's K rows, 32 per pipeline stage
 //              (four warps the A chunks, two warps the B chunks);
 //   warp 6     allocates the tensor memory (6 levels x 64 columns in 512); one
-//              of its threads issues nine MMAs (M=128, K=32, N=64..256) per
+//              of its threads, alone (a vote a stage: 5 % slower at 200 waters),
+//              issues nine MMAs (M=128, K=32, N=64..256) per
 //              stage, one per A digit plane and run of up to four B digit
 //              planes;
 //   warp 7     expands the tiles' inner lists (runs of panel rows) into the 32
@@ -57,14 +58,16 @@
 // in shared memory, and from the row sums, which overwrite the staged columns
 // they came from.  Tiles alone: 200 waters, cutoff 8 (65 stages a tile): 0.73 ->
 // 0.68 ms, 2,850 of the probe's 4,340 TOP/s; 1,536 waters, cutoff 7 (11 stages a
-// tile, bound by the epilogue's ~14 k clocks): 5.54 -> 4.75 ms.  Slower there:
+// tile, bound by the epilogue's ~14 k clocks): 5.54 -> 4.75 ms (4.57 since; the
+// roles' leaving together took 0.5 % of it).  Slower there:
 // storing straight from tensor memory (6.2 ms: it stays occupied), whole blocks
 // by a warp (5.9), eight columns loaded ahead of their stores (6.3).
 // Every wait on an mbarrier is bounded (2 s of %globaltimer); on a timeout
 // the kernel records an error code, every role stops, and the host returns
-// an error status.  The roles stop by whole warps (a wait answers for its warp),
-// the epilogue by all of its warps at one vote a tile: whoever left alone would
-// be missing from the barriers of the others, which have no limit.
+// an error status.  Whoever left a role alone would be missing from the barriers
+// of the others, which have no limit: a producer warp's lanes leave at the vote
+// after a stage's copies, the epilogue's warps at the vote after staging, and the
+// MMA issuer is a single thread.  MMAs and copies in flight are waited for.
 #include <cub/cub.cuh>
 
 #include <algorithm>

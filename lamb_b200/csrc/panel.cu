@@ -20,12 +20,12 @@
 //
 // What bounds it: the FP64 tensor pipe (37.1 TFLOP/s, 16 cycles per m8n8k4).
 // At 6,144 waters (cutoff 8) the multiply's 775 GFLOP took 103 ms in the stack
-// kernel and 22 ms in its fills; here 49 ms and 2.6 ms for the panels (15.8
+// kernel and 22 ms in its fills; here 48 ms and 2.6 ms for the panels (16.1
 // TFLOP/s).  55 to 60 % of the executed MMA work is useful (absent blocks of a
 // superblock, 23 of 24 rows), the pipe is about 70 % busy; the rest is a warp's
 // own serial work per tile (listing, first copies, writing out), which three
 // warps per sub-partition hide only partly.  Tried and slower (768 waters,
-// cutoff 7; now 3.3 ms): fragments straight from global memory 7.9 ms, 4 x 4
+// cutoff 7; now 3.2 ms): fragments straight from global memory 7.9 ms, 4 x 4
 // tiles behind one copy pipeline 7.4 ms (its warps wait for one another), 2 x 2
 // tiles in four such teams 4.3 ms, sixteen warps with rings of 8-row copies
 // 4.5 ms (issue-bound).
@@ -394,8 +394,9 @@ static_assert(kTileSmem <= 232448, "the tile kernel exceeds the shared memory of
 
 // Waits for the phase of the given parity, at most limit_ns; then records
 // `code` and stops the CTA.  The answer is the whole warp's: lanes that left
-// by themselves would be missing from the shuffles of the others.  A limit of
-// 0 counts every wait as run out, without looking.
+// by themselves would be missing from the shuffles of the others (389 waters
+// with 23-row O blocks: 8.39 ms with an answer a lane, 7.93 with the votes).  A
+// limit of 0 counts every wait as run out, without looking.
 __device__ __forceinline__ bool tile_wait(unsigned long long* b, uint32_t parity, uint64_t limit_ns, int* abort,
                                           int* err, int code) {
   if (__all_sync(0xffffffffu, limit_ns != 0 && bar_try(b, parity))) return true;
